@@ -1,0 +1,75 @@
+"""Attention of a few query rows per sequence over cached keys (csrc/attention_cached.cuh) and its tile table."""
+import pytest
+import torch
+
+from wallx_b200.ops import functional as F_
+
+
+def _meta(lq, lk, device, causal, bid, gap=0):
+    """Sequences of ``lq`` new rows against the first ``lk`` rows of key slots that are ``gap`` rows longer."""
+    cu, starts = [0], []
+    for q in lq:
+        cu.append(cu[-1] + q)
+    rows = 0
+    for k in lk:
+        starts.append(rows)
+        rows += k + gap
+    bq = bk = None
+    if bid:
+        bq = torch.arange(cu[-1]) % 3 != 0
+        bk = torch.zeros(rows, dtype=torch.bool)
+        for i, (q, k) in enumerate(zip(lq, lk)):
+            bk[starts[i] + k - q: starts[i] + k] = True
+        bq, bk = bq.to(device), bk.to(device)
+    return F_.AttnMeta(cu, device, causal, bq, bidir_k=bk, k_starts=starts, k_lens=lk, k_rows=rows), rows
+
+
+@pytest.mark.parametrize("causal,bid", [(True, False), (True, True), (False, False)])
+@pytest.mark.parametrize("per_tile", [1, 8, 16, 128])
+def test_tile_table_covers_every_row_and_every_visible_key(causal, bid, per_tile):
+    lq, lk = [1, 31, 16, 17], [1, 200, 16, 90]
+    meta, _ = _meta(lq, lk, "cpu", causal, bid, gap=5)
+    qtab, ktab = meta.device_tables(torch.device("cpu"))
+    seen = []
+    for row0, n, k0, k1 in meta.row_tiles("cpu", per_tile).tolist():
+        assert 1 <= n <= per_tile
+        seen += range(row0, row0 + n)
+        q = qtab[row0: row0 + n]
+        assert (q[:, 0] == k0).all()  # one sequence
+        upper = torch.where(q[:, 3] != 0, q[:, 1], torch.minimum(q[:, 2] + 1, q[:, 1])).max().item()
+        assert upper <= k1 <= q[0, 1].item()
+        if not bid:
+            assert upper == k1
+    assert seen == list(range(sum(lq)))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("causal,bid", [(True, False), (True, True), (False, False)])
+@pytest.mark.parametrize("hq,hkv", [(16, 2), (4, 4), (2, 1), (32, 2)])
+@pytest.mark.parametrize("lq,lk", [([1], [1]), ([1, 1, 1], [127, 128, 129]), ([15, 16, 17], [15, 300, 256]),
+                                   ([33, 2], [1100, 64]), ([128] * 3, [128, 500, 257]), ([5] * 40, [70] * 40)])
+def test_cached_attention_matches_fp32(lq, lk, hq, hkv, causal, bid):
+    """Tile and block edges, group sizes 1 to 16, one to eight CTAs per sequence. The key slots are longer than their valid
+    part and the rest holds NaN: nothing of it may reach a result. The bound is that of the other attention kernels."""
+    torch.manual_seed(5)
+    D = 128
+    meta, rows = _meta(lq, lk, "cuda", causal, bid, gap=3)
+    ref_meta, _ = _meta(lq, lk, "cpu", causal, bid, gap=3)
+    q = torch.randn(sum(lq), hq * D).to(torch.bfloat16)
+    kv = torch.randn(rows, 2 * hkv * D).to(torch.bfloat16)
+    kf = kv.float()
+    want = F_.attention(q.float(), kf[:, : hkv * D], kf[:, hkv * D:], ref_meta, hq, hkv, D)
+    for (k0, k1), nxt in zip(meta.k_ranges, [r[0] for r in meta.k_ranges[1:]] + [rows]):
+        kv[k1:nxt] = float("nan")
+    kv = kv.cuda()
+    with torch.no_grad():
+        got = F_.attention_decode(q.cuda(), kv[:, : hkv * D], kv[:, hkv * D:], meta, hq, hkv, D)
+        again = F_.attention_decode(q.cuda(), kv[:, : hkv * D], kv[:, hkv * D:], meta, hq, hkv, D)
+    torch.cuda.synchronize()
+    from wallx_b200.ops import gemm as G
+
+    G.check_status()
+    assert torch.equal(got, again)
+    # the result is rounded to bf16 (relative 2^-9); scores and sums are fp32, probabilities have 16 significant bits
+    err = (got.float().cpu() - want).abs().max().item()
+    assert err <= 2.0 ** -8 * want.abs().max().item(), err

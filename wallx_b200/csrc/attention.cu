@@ -17,6 +17,7 @@
 // modeling_qwen2_5_vl.py:208-210 and :1008-1015, and the masked eager path of
 // modeling_qwen2_5_vl_act.py:616-637.
 #include "attention.h"
+#include "devinfo.h"
 #include "ptx.cuh"
 
 #include <math.h>
@@ -966,3 +967,5 @@ int attn_bwd(const AttnShape& s, const void* q, const void* k, const void* v, co
 }
 
 }  // namespace wx
+
+#include "attention_cached.cuh"

@@ -30,6 +30,14 @@ int attn_bwd(const AttnShape& s, const void* q, const void* k, const void* v, co
              void* dq, long ld_dq, void* dk, long ld_dk, void* dv, long ld_dv, float* part_k, float* part_v,
              cudaStream_t stream, int* status);
 
+// Few query rows per sequence over a long key range (attention_cached.cuh), head dim 128. `tiles`: int32 [ntiles, 4] =
+// (first query row, rows, first key, end of the keys that some row sees), each tile at most 128 / (hq / hkv) consecutive
+// rows of one sequence, together covering every row. `max_keys`: the longest key range of a query row (0: unknown).
+bool attn_cached_supported(int hq, int hkv, int D);
+int attn_cached(const AttnShape& s, const void* q, const void* k, const void* v, const void* qtab, const void* ktab,
+                const void* tiles, int ntiles, int max_keys, void* out, long ld_out, cudaStream_t stream,
+                int* status);
+
 // Debug build (-DWX_CHECK): this translation unit's range-check record {first violating site, violation count, two
 // values}, cleared when `clear`; all zeros in a release build. Returns a CUDA error code.
 int attn_check_read(long long* out4, int clear);

@@ -1,0 +1,479 @@
+// Attention of a few query rows per sequence over a long key range (denoise and decoding steps against the key-value
+// cache), sm_100a. Included by attention.cu after the general kernels; same tables, same masking rule.
+//
+// What bounds such a step is latency. The general forward kernel gives a CTA 128 consecutive query rows of ONE head: with
+// 32 new rows per sequence its tiles span several sequences, walk the keys of all of them one 64-key block after the
+// other, and read every key once per query head. Here a CTA's 128 accumulator rows are the query heads that share one
+// key-value head times consecutive rows of ONE sequence (8 heads x 16 rows at 16 / 2 heads: a 3-D tensor map delivers
+// them in that order), so keys and values are read once per group, a tile never sees another sequence's keys, and the
+// 128-key blocks of the sequence are dealt to the CTAs of a cluster: one block per CTA at the usual lengths, so the
+// whole call is one QK^T, one softmax, one PV and a merge of the partial results through distributed shared memory in
+// split order (results do not depend on timing).
+//
+// The probabilities enter the second product as the sum of two bf16 values (16 significant bits): calls of up to 128 rows
+// had fp32 probabilities in the kernel that served them before, and the error against 64 bits stays the same, 1.66e-3 at
+// 32 x 346 (the rounding of the result); one bf16 value gives 2.15e-3.
+//
+// Two threads per accumulator row (64 of the block's 128 keys each): with one, the exponentials of a block took as long as
+// everything else together. Shared memory holds two key / value stages, so a CTA with several blocks loads the next one and
+// runs its QK^T while the softmax of the current one is under way.
+//
+// Measured (B200, 16 / 2 heads of 128, us per call in a CUDA graph; before = the faster of the other two kernels that could
+// serve the call):
+//   rows x keys (sequences)   before   now
+//   1 x 346 (1)                9.0      8.6
+//   32 x 346 (1)              13.7     10.3
+//   155 x 310..327 (5)        53.6     10.8
+//   1024 x 346 (32)           45.4     13.3
+//   64 x 900 (1)              30.6     12.1
+//   1024 x 900 (8)            32.1     23.2
+// What is left of a one-block call is latency: launch, tensor memory and barriers 3 us, table and TMA 2 us, the rest the
+// two products, the softmax and the merge.
+#pragma once
+
+#include "launch.h"
+
+#include <atomic>
+
+namespace wx {
+namespace {
+
+constexpr int kCachedThreads = 288;    // 8 softmax warps (two threads per accumulator row), 1 issue warp
+constexpr int kCachedBlock = 128;      // keys per block
+constexpr int kCachedMaxSplits = 8;    // portable cluster size
+constexpr int kCachedPitch = 132;      // floats per row of a partial result (16-byte accesses without bank conflicts)
+
+struct CachedArgs {
+  CUtensorMap tmQ;  // 3-D: channel, head, row; box {64, rep, 128 / rep}
+  CUtensorMap tmK;  // box {64, 128}
+  CUtensorMap tmV;
+  const int4* tiles;  // per tile: first query row, rows (<= 128 / rep, all of one sequence), first key, end of visible keys
+  const int4* qtab;
+  const int4* ktab;
+  __nv_bfloat16* out;
+  long ld_out;
+  int Tq, Tk, rep;
+  float scale_log2;
+  int has_bidir;
+  int splits;
+};
+
+constexpr int kCachedQ = 0;            // two [128][64] tiles
+constexpr int kCachedStage0 = 32768;   // stage s: K (two [128][64] tiles), then V; the high parts of P overwrite K
+constexpr int kCachedStage = 65536;
+constexpr int kCachedPlo = kCachedStage0 + 2 * kCachedStage;
+constexpr int kCachedSmem = kCachedPlo + 32768 + 1024;
+static_assert(128 * kCachedPitch * 4 <= kCachedPlo, "the partial result reuses the operand tiles");
+
+__global__ void __launch_bounds__(kCachedThreads, 1)
+attn_cached_kernel(const __grid_constant__ CachedArgs a, int* __restrict__ status) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  __shared__ uint64_t bar[8];
+  __shared__ uint32_t tmem_slot;
+  __shared__ int s_abort;
+  __shared__ float s_max[2][2][128];  // [block parity][key half][row]
+  __shared__ float4 s_ml[2][128];     // (m, l) of every row and key half
+  __shared__ float s_w[kCachedMaxSplits][128];
+  uint64_t* qk_full = &bar[0];  // [2]
+  uint64_t* v_full = &bar[2];   // [2]
+  uint64_t* s_bar = &bar[4];    // [2]
+  uint64_t* p_ready = &bar[6];
+  uint64_t* pv_bar = &bar[7];
+  volatile int* abort_flag = &s_abort;
+
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const bool is_row = warp < 8;
+  const int splits = a.splits;
+  const int tile_idx = static_cast<int>(blockIdx.x) / splits;
+  const int split = static_cast<int>(blockIdx.x) - tile_idx * splits;  // = %cluster_ctarank
+  const int g = blockIdx.y;
+  if (tid == 256) {
+    for (int i = 0; i < 8; ++i) mbar_init(&bar[i], i == 6 ? 256 : 1);
+    s_abort = 0;
+    fence_mbar_init();
+    tma_prefetch_desc(&a.tmQ);
+    tma_prefetch_desc(&a.tmK);
+    tma_prefetch_desc(&a.tmV);
+  }
+  if (warp == 0) {
+    tmem_alloc(&tmem_slot, 512);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  pdl_wait();
+  pdl_launch_dependents();
+  const uint32_t tmem = tmem_slot;
+  const uint32_t tO = tmem + 256;  // 128 columns; S of block parity p: 128 columns at tmem + 128 p
+
+  int4 tile = a.tiles[tile_idx];
+  if (!WX_CHK(tile.x >= 0 && tile.y >= 0 && tile.x + tile.y <= a.Tq && tile.y * a.rep <= 128 && tile.z >= 0 && tile.w <= a.Tk, 3101,
+              tile.x, tile.y))
+    tile = make_int4(0, 0, 0, 0);
+  const int kmin = tile.z, kmax = tile.w;
+  const int nblk_all = (kmax > kmin) ? (kmax - kmin + kCachedBlock - 1) / kCachedBlock : 0;
+  const int nblk = nblk_all > split ? (nblk_all - split + splits - 1) / splits : 0;  // this CTA: split, split + splits, ...
+  const int arow = (warp & 3) * 32 + lane;  // accumulator row = row of the tile x rep + head of the group
+  const int half = (warp >> 2) & 1;         // which half of a block's keys, and of the output channels
+  const int r_local = arow / a.rep;
+  const int row = tile.x + r_local;
+  const bool row_ok = is_row && r_local < tile.y;
+  float m_run = -INFINITY, l_run = 0.f;
+  bool ok = nblk > 0;
+
+  if (!is_row) {
+    // ------------------------------------------------------------------ issue warp
+    if (tid == 256 && nblk > 0) {
+      constexpr uint32_t idesc_s = make_idesc_bf16(128, 128, false, false);
+      constexpr uint32_t idesc_o = make_idesc_bf16(128, 128, false, true);
+      const uint32_t qa = smem_u32(smem + kCachedQ), pa = smem_u32(smem + kCachedPlo);
+      auto load = [&](int it) {
+        const int st = it & 1;
+        const int kbase = kmin + (split + it * splits) * kCachedBlock;
+        uint8_t* sK = smem + kCachedStage0 + st * kCachedStage;
+        mbar_arrive_expect_tx(&qk_full[st], it == 0 ? 65536u : 32768u);
+        for (int b = 0; b < 2; ++b) {
+          if (it == 0) tma_load_3d(smem + kCachedQ + b * 16384, &a.tmQ, &qk_full[st], b * 64, g * a.rep, tile.x);
+          tma_load_2d(sK + b * 16384, &a.tmK, &qk_full[st], g * 128 + b * 64, kbase);
+        }
+        mbar_arrive_expect_tx(&v_full[st], 32768u);
+        for (int b = 0; b < 2; ++b) tma_load_2d(sK + 32768 + b * 16384, &a.tmV, &v_full[st], g * 128 + b * 64, kbase);
+      };
+      // O += (P_hi + P_lo) V of block `it`; the next block that this stage holds is requested once it has been read
+      auto pv = [&](int it) {
+        const int st = it & 1;
+        const uint32_t ka = smem_u32(smem + kCachedStage0 + st * kCachedStage), va = ka + 32768;
+        ok = mbar_wait(&v_full[st], (it >> 1) & 1, abort_flag) && mbar_wait(p_ready, it & 1, abort_flag);
+        if (!ok) return;
+        tc_fence_after();
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          const uint64_t dv = make_smem_desc_sw128(va + k * 2048, 16384, 1024);
+          const uint32_t step = (k >> 2) * 16384 + (k & 3) * 32;
+          tc_mma_bf16(tO, make_smem_desc_sw128(ka + step, 16, 1024), dv, idesc_o, (it | k) != 0);
+          tc_mma_bf16(tO, make_smem_desc_sw128(pa + step, 16, 1024), dv, idesc_o, 1u);
+        }
+        tc_commit(pv_bar);
+        if (it + 2 < nblk) {
+          ok = mbar_wait(pv_bar, it & 1, abort_flag);
+          if (ok) load(it + 2);
+        }
+      };
+      load(0);
+      if (nblk > 1) load(1);
+      for (int it = 0; it < nblk && ok; ++it) {
+        const int st = it & 1;
+        const uint32_t ka = smem_u32(smem + kCachedStage0 + st * kCachedStage);
+        ok = mbar_wait(&qk_full[st], (it >> 1) & 1, abort_flag);
+        if (!ok) break;
+        tc_fence_after();
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          const uint32_t step = (k >> 2) * 16384 + (k & 3) * 32;
+          tc_mma_bf16(tmem + st * 128, make_smem_desc_sw128(qa + step, 16, 1024), make_smem_desc_sw128(ka + step, 16, 1024), idesc_s,
+                      k != 0);
+        }
+        tc_commit(&s_bar[st]);
+        if (it > 0) pv(it - 1);
+      }
+      if (ok) pv(nblk - 1);
+    }
+    __syncwarp();
+  } else {
+    // ------------------------------------------------------------------ softmax warps
+    int4 qi = make_int4(0, 0, -1, 0);
+    if (row_ok) qi = a.qtab[row];
+    if (row_ok && !WX_CHK(qi.x >= kmin && qi.x <= qi.y && qi.y <= a.Tk && qi.z < qi.y, 3102, qi.x, qi.y)) qi = make_int4(0, 0, -1, 0);
+    const uint32_t lane_off = static_cast<uint32_t>((warp & 3) * 32) << 16;
+    for (int it = 0; it < nblk; ++it) {
+      const int st = it & 1;
+      const int base = kmin + (split + it * splits) * kCachedBlock;
+      const int kbase = base + half * 64;
+      uint8_t* stage = smem + kCachedStage0 + st * kCachedStage;
+      const bool all_seen = __all_sync(0xffffffffu, kbase >= qi.x && kbase + 63 <= qi.z && kbase + 63 < qi.y);
+      uint64_t km = ~0ull;
+      if (!all_seen) {
+        uint64_t flags = 0;
+        if (a.has_bidir) {
+          const int k0 = kbase + lane, k1 = k0 + 32;
+          const uint32_t lo = __ballot_sync(0xffffffffu, k0 < a.Tk && (a.ktab[k0].w & 1) != 0);
+          const uint32_t hi = __ballot_sync(0xffffffffu, k1 < a.Tk && (a.ktab[k1].w & 1) != 0);
+          flags = (static_cast<uint64_t>(hi) << 32) | lo;
+        }
+        km = row_key_mask(qi, kbase, flags);
+      }
+      if (ok) ok = mbar_wait(&s_bar[st], (it >> 1) & 1, abort_flag);
+      tc_fence_after();
+      float sc[64];
+      {
+        uint32_t r[2][32];
+        tmem_ld_32x32(tmem + st * 128 + lane_off + half * 64, r[0]);
+        tmem_ld_32x32(tmem + st * 128 + lane_off + half * 64 + 32, r[1]);
+        tmem_ld_wait();
+#pragma unroll
+        for (int c = 0; c < 64; ++c) sc[c] = __uint_as_float(r[c >> 5][c & 31]);
+      }
+      if (!all_seen) {
+        const uint32_t km_lo = static_cast<uint32_t>(km), km_hi = static_cast<uint32_t>(km >> 32);
+#pragma unroll
+        for (int c = 0; c < 32; ++c) {
+          sc[c] = (km_lo & (1u << c)) ? sc[c] : -INFINITY;
+          sc[32 + c] = (km_hi & (1u << c)) ? sc[32 + c] : -INFINITY;
+        }
+      }
+      float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+      for (int c = 0; c < 64; ++c) mx[c & 3] = fmaxf(mx[c & 3], sc[c]);
+      s_max[st][half][arow] = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+      asm volatile("bar.sync 1, 256;" ::: "memory");
+      const float raw_max = fmaxf(s_max[st][0][arow], s_max[st][1][arow]);
+      const float m_new = fmaxf(m_run, raw_max * a.scale_log2);
+      const float m_use = (m_new == -INFINITY) ? 0.f : m_new;
+      const float alpha = (m_run == -INFINITY) ? 0.f : ex2_approx(m_run - m_use);
+      float ps[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int c = 0; c < 64; ++c) {
+        sc[c] = ex2_approx(fmaf(sc[c], a.scale_log2, -m_use));
+        ps[c & 3] += sc[c];
+      }
+      l_run = l_run * alpha + ((ps[0] + ps[1]) + (ps[2] + ps[3]));
+      const bool changed = m_new > m_run;
+      m_run = m_new;
+      if (it > 0) {  // PV(it - 1) has read the low parts and must not be adding into O
+        if (ok) ok = mbar_wait(pv_bar, (it - 1) & 1, abort_flag);
+        tc_fence_after();
+        if (__any_sync(0xffffffffu, changed)) {
+#pragma unroll
+          for (int c = 0; c < 2; ++c) {
+            uint32_t r[32];
+            tmem_ld_32x32(tO + lane_off + half * 64 + 32 * c, r);
+            tmem_ld_wait();
+#pragma unroll
+            for (int e = 0; e < 32; ++e) r[e] = __float_as_uint(__uint_as_float(r[e]) * alpha);
+            tmem_st_32x32(tO + lane_off + half * 64 + 32 * c, r);
+          }
+          tmem_st_wait();
+        }
+      }
+      uint8_t* sP = stage + half * 16384;
+      uint8_t* sL = smem + kCachedPlo + half * 16384;
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        uint32_t hi[4], lo[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float p0 = sc[8 * q + 2 * e], p1 = sc[8 * q + 2 * e + 1];
+          const __nv_bfloat162 h = __floats2bfloat162_rn(p0, p1);
+          const float2 hf = __bfloat1622float2(h);
+          hi[e] = *reinterpret_cast<const uint32_t*>(&h);
+          lo[e] = pack_bf16x2(p0 - hf.x, p1 - hf.y);
+        }
+        const uint32_t off = sw128_offset(arow, q);
+        *reinterpret_cast<uint4*>(sP + off) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+        *reinterpret_cast<uint4*>(sL + off) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+      }
+      if (base + kCachedBlock > kmax) {
+        // value rows past the last visible key belong to nobody here (another sequence's slot, or rows not written yet):
+        // a probability of zero times whatever they hold must not reach the sum
+        if (ok) ok = mbar_wait(&v_full[st], (it >> 1) & 1, abort_flag);
+        for (int i = (kmax - base) * 16 + tid; i < kCachedBlock * 16; i += 256) {
+          const int r = i >> 4, piece = i & 15;  // whole 16-byte pieces of a row: the order within it does not matter
+          *reinterpret_cast<uint4*>(stage + 32768 + (piece >> 3) * 16384 + r * 128 + (piece & 7) * 16) = make_uint4(0u, 0u, 0u, 0u);
+        }
+      }
+      fence_proxy_async_smem();
+      tc_fence_before();
+      mbar_arrive(p_ready);
+    }
+    s_ml[half][arow] = make_float4(m_run, l_run, 0.f, 0.f);
+    if (ok && nblk > 0) ok = mbar_wait(pv_bar, (nblk - 1) & 1, abort_flag);
+    tc_fence_after();
+    if (nblk > 0) {
+      // every MMA has read its operands (pv_bar): the partial result takes their place
+      float* prow = reinterpret_cast<float*>(smem) + arow * kCachedPitch + half * 64;
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        uint32_t r[32];
+        tmem_ld_32x32(tO + lane_off + half * 64 + 32 * c, r);
+        tmem_ld_wait();
+        if (row_ok) {
+#pragma unroll
+          for (int q = 0; q < 8; ++q)
+            *reinterpret_cast<uint4*>(prow + 32 * c + 4 * q) = make_uint4(r[4 * q], r[4 * q + 1], r[4 * q + 2], r[4 * q + 3]);
+        }
+      }
+    }
+  }
+
+  __syncthreads();
+  if (splits > 1) {
+    cluster_arrive();
+    cluster_wait();
+  }
+  if (is_row && half == 0) {  // weight of every split's partial result of this row (0: nothing visible there)
+    float w[kCachedMaxSplits];
+    float m_all = -INFINITY, l_all = 0.f;
+    const uint32_t ml = smem_u32(&s_ml[0][arow]);
+#pragma unroll
+    for (int s = 0; s < kCachedMaxSplits; ++s) {
+      w[s] = -INFINITY;
+      if (s < splits) w[s] = ld_cluster_f32x4(mapa_u32(ml, static_cast<uint32_t>(s))).x;  // (both halves hold the same m)
+      m_all = fmaxf(m_all, w[s]);
+    }
+#pragma unroll
+    for (int s = 0; s < kCachedMaxSplits; ++s) {
+      w[s] = (w[s] == -INFINITY) ? 0.f : ex2_approx(w[s] - m_all);
+      if (s < splits) {
+        const uint32_t peer = mapa_u32(ml, static_cast<uint32_t>(s));
+        l_all = fmaf(w[s], ld_cluster_f32x4(peer).y + ld_cluster_f32x4(peer + 128 * 16).y, l_all);
+      }
+    }
+    const float inv = l_all > 0.f ? 1.f / l_all : 0.f;
+#pragma unroll
+    for (int s = 0; s < kCachedMaxSplits; ++s)
+      if (s < splits) s_w[s][arow] = w[s] * inv;
+  }
+  __syncthreads();
+  if (is_row) {
+    // The rows of the tile are dealt to the warps of the cluster, a whole row (512 contiguous bytes of every partial
+    // result) at a time: with a row per thread every lane of a remote load touched another row, and the merge of three
+    // partial results took longer than the rest of the kernel (32 x 346: 13.4 us, now 10.3).
+    const uint32_t pbase = smem_u32(smem) + static_cast<uint32_t>(lane * 16);
+    const int nrows = tile.y * a.rep;
+    auto store = [&](int r, const float4& o) {
+      const int rl = r / a.rep;
+      __nv_bfloat16* orow = a.out + static_cast<long>(tile.x + rl) * a.ld_out + (g * a.rep + (r - rl * a.rep)) * 128;
+      reinterpret_cast<uint2*>(orow)[lane] = make_uint2(pack_bf16x2(o.x, o.y), pack_bf16x2(o.z, o.w));
+    };
+    if (splits == 1) {  // nothing to merge: several rows in flight per warp
+#pragma unroll 4
+      for (int r = warp; r < nrows; r += 8) {
+        const float w = s_w[0][r];
+        float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (w != 0.f) {
+          o = *reinterpret_cast<const float4*>(smem + (r * kCachedPitch + lane * 4) * 4);
+          o.x *= w, o.y *= w, o.z *= w, o.w *= w;
+        }
+        store(r, o);
+      }
+    } else
+    for (int r = split + splits * warp; r < nrows; r += 8 * splits) {
+      float4 v[kCachedMaxSplits];
+      float w[kCachedMaxSplits];
+#pragma unroll
+      for (int s = 0; s < kCachedMaxSplits; ++s) {
+        w[s] = s < splits ? s_w[s][r] : 0.f;
+        v[s] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (w[s] != 0.f) v[s] = ld_cluster_f32x4(mapa_u32(pbase + r * (kCachedPitch * 4), static_cast<uint32_t>(s)));
+      }
+      float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int s = 0; s < kCachedMaxSplits; ++s) {
+        o.x = fmaf(w[s], v[s].x, o.x);
+        o.y = fmaf(w[s], v[s].y, o.y);
+        o.z = fmaf(w[s], v[s].z, o.z);
+        o.w = fmaf(w[s], v[s].w, o.w);
+      }
+      store(r, o);
+    }
+  }
+  if (splits > 1) {
+    __syncthreads();
+    cluster_arrive();  // nobody leaves while a peer may still read its partial result
+    cluster_wait();
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (tid == 0 && s_abort) atomicExch(status, 5);
+  if (warp == 0) {
+    tc_fence_after();
+    tmem_dealloc(tmem, 512);
+  }
+}
+
+bool tmap_q3d(CUtensorMap* out, const void* ptr, int hq, int rows, long pitch, int rep) {
+  EncodeTiledFn fn = encode_fn();
+  if (!fn) return false;
+  cuuint64_t dims[3] = {128, static_cast<cuuint64_t>(hq), static_cast<cuuint64_t>(rows)};
+  cuuint64_t strides[2] = {256, static_cast<cuuint64_t>(pitch) * 2};
+  cuuint32_t box[3] = {64, static_cast<cuuint32_t>(rep), static_cast<cuuint32_t>(128 / rep)};
+  cuuint32_t es[3] = {1, 1, 1};
+  return fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(ptr), dims, strides, box, es,
+            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// Clusters of `splits` CTAs of the kernel that the device holds at once.
+int cached_capacity(int splits) {
+  static std::atomic<int> cap[kCachedMaxSplits + 1];
+  int n = cap[splits].load(std::memory_order_relaxed);
+  if (n != 0) return n;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(splits * sm_count()));
+  cfg.blockDim = dim3(kCachedThreads);
+  cfg.dynamicSmemBytes = kCachedSmem;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = static_cast<unsigned>(splits);
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  if (cudaOccupancyMaxActiveClusters(&n, attn_cached_kernel, &cfg) != cudaSuccess) {
+    cudaGetLastError();
+    n = 0;
+  }
+  if (n < 1) n = -1;  // cannot be scheduled: never chosen
+  cap[splits].store(n, std::memory_order_relaxed);
+  return n;
+}
+
+}  // namespace
+
+bool attn_cached_supported(int hq, int hkv, int D) {
+  if (D != 128 || hkv < 1 || hq % hkv != 0) return false;
+  const int rep = hq / hkv;
+  return rep <= 128 && (rep & (rep - 1)) == 0;  // the group's heads divide the 128 accumulator rows
+}
+
+int attn_cached(const AttnShape& s, const void* q, const void* k, const void* v, const void* qtab, const void* ktab,
+                const void* tiles, int ntiles, int max_keys, void* out, long ld_out, cudaStream_t stream,
+                int* status) {
+  if (!attn_cached_supported(s.hq, s.hkv, s.D) || s.ld_q % 8 || s.ld_k % 8 || s.ld_v % 8 || ld_out % 8) return -1;
+  if (s.Tq == 0 || ntiles == 0) return 0;
+  CachedArgs a{};
+  a.rep = s.hq / s.hkv;
+  // (tmap2d first: it binds the calling thread's context for the encode calls)
+  if (!tmap2d(&a.tmK, k, static_cast<uint64_t>(s.hkv) * 128, s.Tk, s.ld_k, kCachedBlock)) return -2;
+  if (!tmap2d(&a.tmV, v, static_cast<uint64_t>(s.hkv) * 128, s.Tk, s.ld_v, kCachedBlock)) return -2;
+  if (!tmap_q3d(&a.tmQ, q, s.hq, s.Tq, s.ld_q, a.rep)) return -2;
+  a.tiles = reinterpret_cast<const int4*>(tiles);
+  a.qtab = reinterpret_cast<const int4*>(qtab);
+  a.ktab = reinterpret_cast<const int4*>(ktab);
+  a.out = reinterpret_cast<__nv_bfloat16*>(out);
+  a.ld_out = ld_out;
+  a.Tq = s.Tq;
+  a.Tk = s.Tk;
+  a.scale_log2 = s.scale * LOG2E;
+  a.has_bidir = s.has_bidir;
+  static bool attr = false;
+  if (!attr) {
+    cudaError_t e = cudaFuncSetAttribute(attn_cached_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kCachedSmem);
+    if (e != cudaSuccess) return static_cast<int>(e);
+    attr = true;
+  }
+  // One CTA per key block of the longest sequence while all clusters are resident at once: a second wave costs more than a
+  // second block in the same CTA (128 rows x 900 keys: 22.8 us with 16 clusters of 8, of which the device holds fewer).
+  const int keys = max_keys > 0 && max_keys < s.Tk ? max_keys : s.Tk;
+  const int blocks = (keys + kCachedBlock - 1) / kCachedBlock;
+  int splits = blocks < kCachedMaxSplits ? blocks : kCachedMaxSplits;
+  while (splits > 1 && cached_capacity(splits) < ntiles * s.hkv) --splits;
+  if (splits < 1) splits = 1;
+  a.splits = splits;
+  return static_cast<int>(launch_kernel_cluster(attn_cached_kernel,
+                                                dim3(static_cast<unsigned>(ntiles * splits), static_cast<unsigned>(s.hkv)),
+                                                dim3(kCachedThreads), kCachedSmem, stream, static_cast<unsigned>(splits), a, status));
+}
+
+}  // namespace wx

@@ -210,6 +210,22 @@ std::tuple<at::Tensor, at::Tensor> attn_fwd(const at::Tensor& q, const at::Tenso
   return {out, lse};
 }
 
+at::Tensor attn_cached(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const at::Tensor& qtab,
+                       const at::Tensor& ktab, const at::Tensor& tiles, int64_t hq, int64_t hkv, int64_t d, double scale,
+                       bool has_bidir, int64_t max_keys) {
+  wx::AttnShape s = attn_shape(q, k, v, hq, hkv, d, scale, has_bidir, false);
+  TORCH_CHECK(qtab.scalar_type() == at::kInt && qtab.is_contiguous() && qtab.size(0) == s.Tq && qtab.size(1) == 4);
+  TORCH_CHECK(ktab.scalar_type() == at::kInt && ktab.is_contiguous() && ktab.size(0) == s.Tk && ktab.size(1) == 4);
+  TORCH_CHECK(tiles.is_cuda() && tiles.scalar_type() == at::kInt && tiles.is_contiguous() && tiles.dim() == 2 && tiles.size(1) == 4);
+  c10::cuda::CUDAGuard guard(q.device());
+  at::Tensor out = at::empty({s.Tq, hq * d}, q.options());
+  int rc = wx::attn_cached(s, q.data_ptr(), k.data_ptr(), v.data_ptr(), qtab.data_ptr(), ktab.data_ptr(), tiles.data_ptr(),
+                           static_cast<int>(tiles.size(0)), static_cast<int>(max_keys), out.data_ptr(), out.stride(0),
+                           at::cuda::getCurrentCUDAStream(), status_tensor(q.device()).data_ptr<int>());
+  TORCH_CHECK(rc == 0, "attn_cached failed with code ", rc);
+  return out;
+}
+
 // dq / dk / dv are written in place into caller-provided (possibly strided) views.
 void attn_bwd(const at::Tensor& dout, const at::Tensor& q, const at::Tensor& k, const at::Tensor& v,
               const at::Tensor& out, const at::Tensor& lse, const at::Tensor& qtab, const at::Tensor& ktab,
@@ -273,6 +289,10 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   }, "the device-side status words themselves (int32[4]; word 0 non-zero after a wait ran out)");
   m.def("attn_fwd", &attn_fwd);
   m.def("attn_bwd", &attn_bwd);
+  m.def("attn_cached", &attn_cached);
+  m.def("attn_cached_supported", [](int64_t hq, int64_t hkv, int64_t d) {
+    return wx::attn_cached_supported(static_cast<int>(hq), static_cast<int>(hkv), static_cast<int>(d));
+  });
   register_kernel_bindings(m);
   register_block_bindings(m);
 }

@@ -119,6 +119,15 @@ __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* t
       "l"(tmap), "r"(smem_u32(bar)), "r"(c0), "r"(c1)
       : "memory");
 }
+// 3-D tiled load (c0 innermost: the 16-byte rule of tma_load_2d)
+__device__ __forceinline__ void tma_load_3d(void* smem_dst, const CUtensorMap* tmap, uint64_t* bar, int c0, int c1, int c2) {
+  if (!WX_CHK((c0 & 7) == 0 && (smem_u32(smem_dst) & 127u) == 0u, 1009, c0, c1)) return;
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes"
+      " [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(smem_u32(smem_dst)),
+      "l"(tmap), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2)
+      : "memory");
+}
 __device__ __forceinline__ void tma_store_2d(const CUtensorMap* tmap, const void* smem_src, int c0,
                                              int c1) {
   if (!WX_CHK((c0 & 7) == 0 && c0 >= 0 && c1 >= 0, 1003, c0, c1)) return;  // stores never start at a negative coordinate

@@ -606,6 +606,22 @@ class AttnMeta:
     def cu_host(self):
         return self.cu_q_host
 
+    def row_tiles(self, device, rows_per_tile: int) -> torch.Tensor:
+        """int32 ``[n, 4]`` (first query row, rows, first key, end of the keys that some row sees): every sequence's
+        queries cut into tiles of up to ``rows_per_tile`` rows."""
+        t = self._dev.get(("tiles", rows_per_tile))
+        if t is None:
+            cu = self.cu_q_host
+            causal = self.causal and not _attn_flags(self)[0]
+            t = []
+            for i, (k0, k1) in enumerate(self.k_ranges):
+                for r in range(cu[i], cu[i + 1], rows_per_tile):
+                    e = min(r + rows_per_tile, cu[i + 1])
+                    t.append((r, e - r, k0, max(k0, k1 - (cu[i + 1] - e)) if causal else k1))
+            t = torch.tensor(t, dtype=torch.int32).reshape(-1, 4).to(device)
+            self._dev[("tiles", rows_per_tile)] = t
+        return t
+
     def device_tables(self, device):
         """Per-token tables for the kernels: for every query row its key range and causal limit."""
         t = self._dev.get("tables")
@@ -759,6 +775,8 @@ def attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, meta: AttnMeta,
     return _attention_torch(q, k, v, meta, hq, hkv, d, scale)
 
 
+CACHED_MAX_ROWS = 128  # query rows of a sequence up to which a cached step runs on the cached kernel (8 x 128 rows, 900
+# keys: 23 against 32 us for the general kernel; longer calls are prefix passes)
 DECODE_MAX_ROWS = 128  # query rows up to which the cached step uses the small-query attention kernel
 
 
@@ -780,10 +798,15 @@ def rope_cache_(qkv: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, cache_r
 
 def attention_decode(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, meta: AttnMeta, hq: int, hkv: int, d: int,
                      scale: Optional[float] = None) -> torch.Tensor:
-    """:func:`attention` for a handful of query rows over a long cached key range (decode and denoise steps): one CTA
-    per query row and key-value head with the keys staged in shared memory (csrc/decode.cu). Inference only; falls
-    back to :func:`attention` for shapes the kernel does not serve."""
+    """:func:`attention` for a handful of query rows per sequence over a long cached key range (decode and denoise steps):
+    the tensor-core kernel of csrc/attention_cached.cuh, or csrc/decode.cu where the heads of a group do not divide its
+    128 rows. Inference only; falls back to :func:`attention` for shapes neither kernel serves."""
     scale = scale if scale is not None else 1.0 / math.sqrt(d)
+    if (_is_cuda(q) and not torch.is_grad_enabled() and 0 < meta.max_q <= CACHED_MAX_ROWS
+            and _C().attn_cached_supported(hq, hkv, d)):
+        qtab, ktab = meta.device_tables(q.device)
+        return _C().attn_cached(q, k, v, qtab, ktab, meta.row_tiles(q.device, 128 // (hq // hkv)), int(hq), int(hkv), int(d),
+                                float(scale), _attn_flags(meta)[0], int(meta.max_k))
     if not (_is_cuda(q) and not torch.is_grad_enabled() and q.shape[0] <= DECODE_MAX_ROWS
             and _C().attn_decode_supported(q.shape[0], hq, hkv, d)):
         return attention(q, k, v, meta, hq, hkv, d, scale)
