@@ -116,7 +116,7 @@ attn_fwd_kernel(const __grid_constant__ AttnArgs a, int* __restrict__ status) {
   uint64_t* p_ready = &ctl.bar[6];
   volatile int* abort_flag = &ctl.abort_flag;
 
-  const int tid = threadIdx.x, warp = tid >> 5;
+  const int tid = threadIdx.x, warp = warp_index();
   const bool is_row = warp < 4;
   const int h = blockIdx.y;
   const int g = h / (a.hq / a.hkv);
@@ -163,55 +163,60 @@ attn_fwd_kernel(const __grid_constant__ AttnArgs a, int* __restrict__ status) {
 
   if (!is_row) {
     // ------------------------------------------------------------------ issue warp
-    if (tid == 128 && nblk > 0) {
+    // (one elected lane issues, the whole warp runs the loop: descriptors and coordinates stay in uniform registers)
+    const int n = warp_uniform(nblk), k_first = warp_uniform(kmin);
+    const uint32_t tSu = warp_uniform(tS), tOu = warp_uniform(tO);
+    if (n > 0) {
       const uint32_t kv_bytes = static_cast<uint32_t>(nbox) * 8192u * 2u;
       const uint32_t idesc_s = make_idesc_bf16(128, 64, false, false);
       const uint32_t idesc_o = make_idesc_bf16(128, D, false, true);
+      const uint64_t dq = make_smem_desc_sw128(smem_u32(sQ), 16, 1024);
+      const uint64_t dk0 = make_smem_desc_sw128(smem_u32(sKV), 16, 1024);  // K stage 0; P takes its place
+      const uint64_t dv0 = make_smem_desc_sw128(smem_u32(sKV) + 16384, 8192, 1024);
       auto load_kv = [&](int j) {
         const int st = j & 1;
         uint8_t* sK = sKV + st * 32768;
         uint8_t* sV = sK + 16384;
         mbar_arrive_expect_tx(&kv_full[st], kv_bytes);
         for (int b = 0; b < nbox; ++b) {
-          tma_load_2d(sK + b * 8192, &a.tmK, &kv_full[st], g * D + b * 64, kmin + j * 64);
-          tma_load_2d(sV + b * 8192, &a.tmV, &kv_full[st], g * D + b * 64, kmin + j * 64);
+          tma_load_2d(sK + b * 8192, &a.tmK, &kv_full[st], g * D + b * 64, k_first + j * 64);
+          tma_load_2d(sV + b * 8192, &a.tmV, &kv_full[st], g * D + b * 64, k_first + j * 64);
         }
       };
-      mbar_arrive_expect_tx(q_full, static_cast<uint32_t>(nbox) * 16384u);
-      for (int b = 0; b < nbox; ++b) tma_load_2d(sQ + b * 16384, &a.tmQ, q_full, h * D + b * 64, r0);
-      load_kv(0);
-      if (nblk > 1) load_kv(1);
-      ok = mbar_wait(q_full, 0, abort_flag);
-      const uint32_t qa = smem_u32(sQ);
-      for (int j = 0; j < nblk && ok; ++j) {
+      if (elect_one()) {
+        mbar_arrive_expect_tx(q_full, static_cast<uint32_t>(nbox) * 16384u);
+        for (int b = 0; b < nbox; ++b) tma_load_2d(sQ + b * 16384, &a.tmQ, q_full, h * D + b * 64, r0);
+        load_kv(0);
+        if (n > 1) load_kv(1);
+      }
+      ok = __all_sync(0xffffffffu, mbar_wait(q_full, 0, abort_flag));
+      for (int j = 0; j < n && ok; ++j) {
         const int st = j & 1;
-        const uint32_t ka = smem_u32(sKV + st * 32768), va = ka + 16384;
+        const uint64_t dk = dk0 + st * 2048, dv = dv0 + st * 2048;
         ok = mbar_wait(&kv_full[st], (j >> 1) & 1, abort_flag);
         if (ok && j > 0) ok = mbar_wait(s_free, (j - 1) & 1, abort_flag);  // S(j-1) is in registers
+        ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         tc_fence_after();
-        for (int k = 0; k < D / 16; ++k) {
-          const uint64_t da = make_smem_desc_sw128(qa + (k >> 2) * 16384 + (k & 3) * 32, 16, 1024);
-          const uint64_t db = make_smem_desc_sw128(ka + (k >> 2) * 8192 + (k & 3) * 32, 16, 1024);
-          tc_mma_bf16(tS, da, db, idesc_s, k != 0);
+        if (elect_one()) {
+          for (int k = 0; k < D / 16; ++k)
+            tc_mma_bf16(tSu, dq + (k >> 2) * 1024 + (k & 3) * 2, dk + (k >> 2) * 512 + (k & 3) * 2, idesc_s, k != 0);
+          tc_commit(s_bar);
         }
-        tc_commit(s_bar);
         // stage (j+1)&1 was last read by PV(j-1): refill it once that is done
-        if (j > 0 && j + 1 < nblk) {
-          ok = mbar_wait(pv_bar, (j - 1) & 1, abort_flag);
+        if (j > 0 && j + 1 < n) {
+          ok = __all_sync(0xffffffffu, mbar_wait(pv_bar, (j - 1) & 1, abort_flag));
           if (!ok) break;
-          load_kv(j + 1);
+          if (elect_one()) load_kv(j + 1);
         }
-        ok = mbar_wait(p_ready, j & 1, abort_flag);
+        ok = __all_sync(0xffffffffu, mbar_wait(p_ready, j & 1, abort_flag));
         if (!ok) break;
         tc_fence_after();
+        if (elect_one()) {
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const uint64_t da = make_smem_desc_sw128(ka + k * 32, 16, 1024);          // P lives in the K stage
-          const uint64_t db = make_smem_desc_sw128(va + k * 2048, 8192, 1024);
-          tc_mma_bf16(tO, da, db, idesc_o, (j | k) != 0);
+          for (int k = 0; k < 4; ++k) tc_mma_bf16(tOu, dk + 2 * k, dv + 128 * k, idesc_o, (j | k) != 0);  // P lives in the K stage
+          tc_commit(pv_bar);
         }
-        tc_commit(pv_bar);
       }
     }
   } else {
@@ -379,7 +384,7 @@ attn_dq_kernel(const __grid_constant__ AttnArgs a, int* __restrict__ status) {
   uint64_t* ds_ready = &ctl.bar[4];
   volatile int* abort_flag = &ctl.abort_flag;
 
-  const int tid = threadIdx.x, warp = tid >> 5;
+  const int tid = threadIdx.x, warp = warp_index();
   const bool is_row = warp < 4;
   const int h = blockIdx.y;
   const int g = h / (a.hq / a.hkv);
@@ -426,50 +431,54 @@ attn_dq_kernel(const __grid_constant__ AttnArgs a, int* __restrict__ status) {
   bool ok = nblk > 0;
 
   if (!is_row) {
-    if (tid == 128 && nblk > 0) {
+    const int n = warp_uniform(nblk), k_first = warp_uniform(kmin);
+    const uint32_t tSu = warp_uniform(tS), tDPu = tSu + 64, tDQu = tSu + 128;
+    if (n > 0) {
       const uint32_t kv_bytes = static_cast<uint32_t>(nbox) * 8192u * 2u;
       const uint32_t idesc_s = make_idesc_bf16(128, 64, false, false);
       const uint32_t idesc_dq = make_idesc_bf16(128, D, false, true);
       auto load_kv = [&](int j) {
         mbar_arrive_expect_tx(kv_full, kv_bytes);
         for (int b = 0; b < nbox; ++b) {
-          tma_load_2d(sK + b * 8192, &a.tmK, kv_full, g * D + b * 64, kmin + j * 64);
-          tma_load_2d(sV + b * 8192, &a.tmV, kv_full, g * D + b * 64, kmin + j * 64);
+          tma_load_2d(sK + b * 8192, &a.tmK, kv_full, g * D + b * 64, k_first + j * 64);
+          tma_load_2d(sV + b * 8192, &a.tmV, kv_full, g * D + b * 64, k_first + j * 64);
         }
       };
-      mbar_arrive_expect_tx(q_full, static_cast<uint32_t>(nbox) * 16384u * 2u);
-      for (int b = 0; b < nbox; ++b) {
-        tma_load_2d(sQ + b * 16384, &a.tmQ, q_full, h * D + b * 64, r0);
-        tma_load_2d(sDO + b * 16384, &a.tmDO, q_full, h * D + b * 64, r0);
+      if (elect_one()) {
+        mbar_arrive_expect_tx(q_full, static_cast<uint32_t>(nbox) * 16384u * 2u);
+        for (int b = 0; b < nbox; ++b) {
+          tma_load_2d(sQ + b * 16384, &a.tmQ, q_full, h * D + b * 64, r0);
+          tma_load_2d(sDO + b * 16384, &a.tmDO, q_full, h * D + b * 64, r0);
+        }
+        load_kv(0);
       }
-      load_kv(0);
-      ok = mbar_wait(q_full, 0, abort_flag);
-      const uint32_t qa = smem_u32(sQ), da_ = smem_u32(sDO), ka = smem_u32(sK), va = smem_u32(sV);
-      for (int j = 0; j < nblk && ok; ++j) {
-        ok = mbar_wait(kv_full, j & 1, abort_flag);
+      ok = __all_sync(0xffffffffu, mbar_wait(q_full, 0, abort_flag));
+      const uint64_t dq = make_smem_desc_sw128(smem_u32(sQ), 16, 1024), ddo = make_smem_desc_sw128(smem_u32(sDO), 16, 1024);
+      const uint64_t dk = make_smem_desc_sw128(smem_u32(sK), 16, 1024), dv = make_smem_desc_sw128(smem_u32(sV), 16, 1024);
+      const uint64_t dkt = make_smem_desc_sw128(smem_u32(sK), 8192, 1024);  // K as the MN-major operand of dS K
+      for (int j = 0; j < n && ok; ++j) {
+        ok = __all_sync(0xffffffffu, mbar_wait(kv_full, j & 1, abort_flag));
         if (!ok) break;
         tc_fence_after();
-        for (int k = 0; k < D / 16; ++k) {
-          const uint32_t ao = (k >> 2) * 16384 + (k & 3) * 32, bo = (k >> 2) * 8192 + (k & 3) * 32;
-          tc_mma_bf16(tS, make_smem_desc_sw128(qa + ao, 16, 1024), make_smem_desc_sw128(ka + bo, 16, 1024), idesc_s, k != 0);
+        if (elect_one()) {
+          for (int k = 0; k < D / 16; ++k)
+            tc_mma_bf16(tSu, dq + (k >> 2) * 1024 + (k & 3) * 2, dk + (k >> 2) * 512 + (k & 3) * 2, idesc_s, k != 0);
+          for (int k = 0; k < D / 16; ++k)
+            tc_mma_bf16(tDPu, ddo + (k >> 2) * 1024 + (k & 3) * 2, dv + (k >> 2) * 512 + (k & 3) * 2, idesc_s, k != 0);
+          tc_commit(s_bar);
         }
-        for (int k = 0; k < D / 16; ++k) {
-          const uint32_t ao = (k >> 2) * 16384 + (k & 3) * 32, bo = (k >> 2) * 8192 + (k & 3) * 32;
-          tc_mma_bf16(tDP, make_smem_desc_sw128(da_ + ao, 16, 1024), make_smem_desc_sw128(va + bo, 16, 1024), idesc_s, k != 0);
-        }
-        tc_commit(s_bar);
-        ok = mbar_wait(ds_ready, j & 1, abort_flag);  // dS is in smem (over V)
+        ok = __all_sync(0xffffffffu, mbar_wait(ds_ready, j & 1, abort_flag));  // dS is in smem (over V)
         if (!ok) break;
         tc_fence_after();
+        if (elect_one()) {
 #pragma unroll
-        for (int k = 0; k < 4; ++k)
-          tc_mma_bf16(tDQ, make_smem_desc_sw128(va + k * 32, 16, 1024), make_smem_desc_sw128(ka + k * 2048, 8192, 1024),
-                      idesc_dq, (j | k) != 0);
-        tc_commit(dq_bar);
-        if (j + 1 < nblk) {  // K and dS are read by the MMA just issued: refill when it is done
-          ok = mbar_wait(dq_bar, j & 1, abort_flag);
+          for (int k = 0; k < 4; ++k) tc_mma_bf16(tDQu, dv + 2 * k, dkt + 128 * k, idesc_dq, (j | k) != 0);
+          tc_commit(dq_bar);
+        }
+        if (j + 1 < n) {  // K and dS are read by the MMA just issued: refill when it is done
+          ok = __all_sync(0xffffffffu, mbar_wait(dq_bar, j & 1, abort_flag));
           if (!ok) break;
-          load_kv(j + 1);
+          if (elect_one()) load_kv(j + 1);
         }
       }
     }
@@ -581,7 +590,7 @@ attn_dkdv_kernel(const __grid_constant__ AttnArgs a, int* __restrict__ status) {
   uint64_t* pt_ready = &ctl.bar[6];
   volatile int* abort_flag = &ctl.abort_flag;
 
-  const int tid = threadIdx.x, warp = tid >> 5;
+  const int tid = threadIdx.x, warp = warp_index();
   const bool is_row = warp < 4;
   const int rep = a.hq / a.hkv;
   const int g = blockIdx.y / rep;
@@ -628,7 +637,9 @@ attn_dkdv_kernel(const __grid_constant__ AttnArgs a, int* __restrict__ status) {
   bool ok = nblk > 0;
 
   if (!is_row) {
-    if (tid == 128 && nblk > 0) {
+    const int n = warp_uniform(nblk), q_first = warp_uniform(qmin);
+    const uint32_t tSu = warp_uniform(tS), tDPu = tSu + 64, tDVu = tSu + 128, tDKu = tSu + 256;
+    if (n > 0) {
       const uint32_t qd_bytes = static_cast<uint32_t>(nbox) * 8192u * 2u;
       const uint32_t idesc_s = make_idesc_bf16(128, 64, false, false);
       const uint32_t idesc_acc = make_idesc_bf16(128, D, false, true);
@@ -638,52 +649,54 @@ attn_dkdv_kernel(const __grid_constant__ AttnArgs a, int* __restrict__ status) {
         uint8_t* d = q + 16384;
         mbar_arrive_expect_tx(&qd_full[st], qd_bytes);
         for (int b = 0; b < nbox; ++b) {
-          tma_load_2d(q + b * 8192, &a.tmQ, &qd_full[st], h * D + b * 64, qmin + i * 64);
-          tma_load_2d(d + b * 8192, &a.tmDO, &qd_full[st], h * D + b * 64, qmin + i * 64);
+          tma_load_2d(q + b * 8192, &a.tmQ, &qd_full[st], h * D + b * 64, q_first + i * 64);
+          tma_load_2d(d + b * 8192, &a.tmDO, &qd_full[st], h * D + b * 64, q_first + i * 64);
         }
       };
-      mbar_arrive_expect_tx(kv_full, static_cast<uint32_t>(nbox) * 16384u * 2u);
-      for (int b = 0; b < nbox; ++b) {
-        tma_load_2d(sK + b * 16384, &a.tmK, kv_full, g * D + b * 64, c0);
-        tma_load_2d(sV + b * 16384, &a.tmV, kv_full, g * D + b * 64, c0);
+      if (elect_one()) {
+        mbar_arrive_expect_tx(kv_full, static_cast<uint32_t>(nbox) * 16384u * 2u);
+        for (int b = 0; b < nbox; ++b) {
+          tma_load_2d(sK + b * 16384, &a.tmK, kv_full, g * D + b * 64, c0);
+          tma_load_2d(sV + b * 16384, &a.tmV, kv_full, g * D + b * 64, c0);
+        }
+        load_qd(0);
+        if (n > 1) load_qd(1);
       }
-      load_qd(0);
-      if (nblk > 1) load_qd(1);
-      ok = mbar_wait(kv_full, 0, abort_flag);
-      const uint32_t ka = smem_u32(sK), va = smem_u32(sV), pa = smem_u32(sPT), sa = smem_u32(sDST);
-      for (int i = 0; i < nblk && ok; ++i) {
+      ok = __all_sync(0xffffffffu, mbar_wait(kv_full, 0, abort_flag));
+      const uint64_t dk = make_smem_desc_sw128(smem_u32(sK), 16, 1024), dv = make_smem_desc_sw128(smem_u32(sV), 16, 1024);
+      const uint64_t dp = make_smem_desc_sw128(smem_u32(sPT), 16, 1024), ds = make_smem_desc_sw128(smem_u32(sDST), 16, 1024);
+      const uint64_t dq0 = make_smem_desc_sw128(smem_u32(sQD), 16, 1024);      // Q of stage 0, dO 16 KB behind it
+      const uint64_t dqt0 = make_smem_desc_sw128(smem_u32(sQD), 8192, 1024);   // the same as MN-major operands
+      for (int i = 0; i < n && ok; ++i) {
         const int st = i & 1;
-        const uint32_t qa = smem_u32(sQD + st * 32768), da_ = qa + 16384;
+        const uint64_t dq = dq0 + st * 2048, ddo = dq + 1024, dqt = dqt0 + st * 2048, ddot = dqt + 1024;
         ok = mbar_wait(&qd_full[st], (i >> 1) & 1, abort_flag);
         if (ok && i > 0) ok = mbar_wait(sp_free, (i - 1) & 1, abort_flag);
+        ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         tc_fence_after();
-        for (int k = 0; k < D / 16; ++k) {
-          const uint32_t ao = (k >> 2) * 16384 + (k & 3) * 32, bo = (k >> 2) * 8192 + (k & 3) * 32;
-          tc_mma_bf16(tS, make_smem_desc_sw128(ka + ao, 16, 1024), make_smem_desc_sw128(qa + bo, 16, 1024), idesc_s, k != 0);
+        if (elect_one()) {
+          for (int k = 0; k < D / 16; ++k)
+            tc_mma_bf16(tSu, dk + (k >> 2) * 1024 + (k & 3) * 2, dq + (k >> 2) * 512 + (k & 3) * 2, idesc_s, k != 0);
+          for (int k = 0; k < D / 16; ++k)
+            tc_mma_bf16(tDPu, dv + (k >> 2) * 1024 + (k & 3) * 2, ddo + (k >> 2) * 512 + (k & 3) * 2, idesc_s, k != 0);
+          tc_commit(s_bar);
         }
-        for (int k = 0; k < D / 16; ++k) {
-          const uint32_t ao = (k >> 2) * 16384 + (k & 3) * 32, bo = (k >> 2) * 8192 + (k & 3) * 32;
-          tc_mma_bf16(tDP, make_smem_desc_sw128(va + ao, 16, 1024), make_smem_desc_sw128(da_ + bo, 16, 1024), idesc_s, k != 0);
-        }
-        tc_commit(s_bar);
-        if (i > 0 && i + 1 < nblk) {  // stage (i+1)&1 was read by the accumulating MMAs of block i-1
-          ok = mbar_wait(acc_bar, (i - 1) & 1, abort_flag);
+        if (i > 0 && i + 1 < n) {  // stage (i+1)&1 was read by the accumulating MMAs of block i-1
+          ok = __all_sync(0xffffffffu, mbar_wait(acc_bar, (i - 1) & 1, abort_flag));
           if (!ok) break;
-          load_qd(i + 1);
+          if (elect_one()) load_qd(i + 1);
         }
-        ok = mbar_wait(pt_ready, i & 1, abort_flag);
+        ok = __all_sync(0xffffffffu, mbar_wait(pt_ready, i & 1, abort_flag));
         if (!ok) break;
         tc_fence_after();
+        if (elect_one()) {
 #pragma unroll
-        for (int k = 0; k < 4; ++k)
-          tc_mma_bf16(tDV, make_smem_desc_sw128(pa + k * 32, 16, 1024), make_smem_desc_sw128(da_ + k * 2048, 8192, 1024),
-                      idesc_acc, (i | k) != 0);
+          for (int k = 0; k < 4; ++k) tc_mma_bf16(tDVu, dp + 2 * k, ddot + 128 * k, idesc_acc, (i | k) != 0);
 #pragma unroll
-        for (int k = 0; k < 4; ++k)
-          tc_mma_bf16(tDK, make_smem_desc_sw128(sa + k * 32, 16, 1024), make_smem_desc_sw128(qa + k * 2048, 8192, 1024),
-                      idesc_acc, (i | k) != 0);
-        tc_commit(acc_bar);
+          for (int k = 0; k < 4; ++k) tc_mma_bf16(tDKu, ds + 2 * k, dqt + 128 * k, idesc_acc, (i | k) != 0);
+          tc_commit(acc_bar);
+        }
       }
     }
   } else {

@@ -82,7 +82,7 @@ attn_cached_kernel(const __grid_constant__ CachedArgs a, int* __restrict__ statu
   uint64_t* pv_bar = &bar[7];
   volatile int* abort_flag = &s_abort;
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
   const bool is_row = warp < 8;
   const int splits = a.splits;
   const int tile_idx = static_cast<int>(blockIdx.x) / splits;
@@ -125,60 +125,72 @@ attn_cached_kernel(const __grid_constant__ CachedArgs a, int* __restrict__ statu
 
   if (!is_row) {
     // ------------------------------------------------------------------ issue warp
-    if (tid == 256 && nblk > 0) {
+    // (one elected lane issues, the whole warp runs the loop: descriptors and coordinates stay in uniform registers)
+    const int n = warp_uniform(nblk), k_first = warp_uniform(kmin), row0 = warp_uniform(tile.x);
+    const uint32_t tSu = warp_uniform(tmem), tOu = tSu + 256;
+    if (n > 0) {
       constexpr uint32_t idesc_s = make_idesc_bf16(128, 128, false, false);
       constexpr uint32_t idesc_o = make_idesc_bf16(128, 128, false, true);
-      const uint32_t qa = smem_u32(smem + kCachedQ), pa = smem_u32(smem + kCachedPlo);
+      const uint64_t dq = make_smem_desc_sw128(smem_u32(smem + kCachedQ), 16, 1024);
+      const uint64_t dlo = make_smem_desc_sw128(smem_u32(smem + kCachedPlo), 16, 1024);
+      const uint64_t dk0 = make_smem_desc_sw128(smem_u32(smem + kCachedStage0), 16, 1024);
+      const uint64_t dv0 = make_smem_desc_sw128(smem_u32(smem + kCachedStage0) + 32768, 16384, 1024);
       auto load = [&](int it) {
         const int st = it & 1;
-        const int kbase = kmin + (split + it * splits) * kCachedBlock;
+        const int kbase = k_first + (split + it * splits) * kCachedBlock;
         uint8_t* sK = smem + kCachedStage0 + st * kCachedStage;
         mbar_arrive_expect_tx(&qk_full[st], it == 0 ? 65536u : 32768u);
+#pragma unroll
         for (int b = 0; b < 2; ++b) {
-          if (it == 0) tma_load_3d(smem + kCachedQ + b * 16384, &a.tmQ, &qk_full[st], b * 64, g * a.rep, tile.x);
+          if (it == 0) tma_load_3d(smem + kCachedQ + b * 16384, &a.tmQ, &qk_full[st], b * 64, g * a.rep, row0);
           tma_load_2d(sK + b * 16384, &a.tmK, &qk_full[st], g * 128 + b * 64, kbase);
         }
         mbar_arrive_expect_tx(&v_full[st], 32768u);
+#pragma unroll
         for (int b = 0; b < 2; ++b) tma_load_2d(sK + 32768 + b * 16384, &a.tmV, &v_full[st], g * 128 + b * 64, kbase);
       };
       // O += (P_hi + P_lo) V of block `it`; the next block that this stage holds is requested once it has been read
       auto pv = [&](int it) {
         const int st = it & 1;
-        const uint32_t ka = smem_u32(smem + kCachedStage0 + st * kCachedStage), va = ka + 32768;
-        ok = mbar_wait(&v_full[st], (it >> 1) & 1, abort_flag) && mbar_wait(p_ready, it & 1, abort_flag);
+        const uint64_t dp = dk0 + st * (kCachedStage >> 4), dv = dv0 + st * (kCachedStage >> 4);
+        ok = __all_sync(0xffffffffu, mbar_wait(&v_full[st], (it >> 1) & 1, abort_flag) && mbar_wait(p_ready, it & 1, abort_flag));
         if (!ok) return;
         tc_fence_after();
+        if (elect_one()) {
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          const uint64_t dv = make_smem_desc_sw128(va + k * 2048, 16384, 1024);
-          const uint32_t step = (k >> 2) * 16384 + (k & 3) * 32;
-          tc_mma_bf16(tO, make_smem_desc_sw128(ka + step, 16, 1024), dv, idesc_o, (it | k) != 0);
-          tc_mma_bf16(tO, make_smem_desc_sw128(pa + step, 16, 1024), dv, idesc_o, 1u);
+          for (int k = 0; k < 8; ++k) {
+            const uint32_t step = (k >> 2) * 1024 + (k & 3) * 2;
+            tc_mma_bf16(tOu, dp + step, dv + 128 * k, idesc_o, (it | k) != 0);
+            tc_mma_bf16(tOu, dlo + step, dv + 128 * k, idesc_o, 1u);
+          }
+          tc_commit(pv_bar);
         }
-        tc_commit(pv_bar);
-        if (it + 2 < nblk) {
-          ok = mbar_wait(pv_bar, it & 1, abort_flag);
-          if (ok) load(it + 2);
+        if (it + 2 < n) {
+          ok = __all_sync(0xffffffffu, mbar_wait(pv_bar, it & 1, abort_flag));
+          if (ok && elect_one()) load(it + 2);
         }
       };
-      load(0);
-      if (nblk > 1) load(1);
-      for (int it = 0; it < nblk && ok; ++it) {
+      if (elect_one()) {
+        load(0);
+        if (n > 1) load(1);
+      }
+      for (int it = 0; it < n && ok; ++it) {
         const int st = it & 1;
-        const uint32_t ka = smem_u32(smem + kCachedStage0 + st * kCachedStage);
-        ok = mbar_wait(&qk_full[st], (it >> 1) & 1, abort_flag);
+        const uint64_t dk = dk0 + st * (kCachedStage >> 4);
+        ok = __all_sync(0xffffffffu, mbar_wait(&qk_full[st], (it >> 1) & 1, abort_flag));
         if (!ok) break;
         tc_fence_after();
+        if (elect_one()) {
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          const uint32_t step = (k >> 2) * 16384 + (k & 3) * 32;
-          tc_mma_bf16(tmem + st * 128, make_smem_desc_sw128(qa + step, 16, 1024), make_smem_desc_sw128(ka + step, 16, 1024), idesc_s,
-                      k != 0);
+          for (int k = 0; k < 8; ++k) {
+            const uint32_t step = (k >> 2) * 1024 + (k & 3) * 2;
+            tc_mma_bf16(tSu + st * 128, dq + step, dk + step, idesc_s, k != 0);
+          }
+          tc_commit(&s_bar[st]);
         }
-        tc_commit(&s_bar[st]);
         if (it > 0) pv(it - 1);
       }
-      if (ok) pv(nblk - 1);
+      if (ok) pv(n - 1);
     }
     __syncwarp();
   } else {

@@ -124,6 +124,19 @@ __device__ __forceinline__ void load_dims(const GemmArgs& args, Dims& d) {
   }
 }
 
+// The sizes may have been read from memory: make them values that the compiler knows to be the same in all lanes.
+__device__ __forceinline__ void make_uniform(Dims& d) {
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    d.M[i] = warp_uniform(d.M[i]);
+    d.K[i] = warp_uniform(d.K[i]);
+    d.m0[i] = warp_uniform(d.m0[i]);
+    d.k0[i] = warp_uniform(d.k0[i]);
+    d.tiles_m[i] = warp_uniform(d.tiles_m[i]);
+    d.tiles[i] = warp_uniform(d.tiles[i]);
+  }
+}
+
 __device__ __forceinline__ TileInfo decode_tile(const Dims& d, int t, bool gathered = false, int rot0 = 0, int rot1 = 0) {
   TileInfo ti;
   ti.prob = 0;
@@ -510,7 +523,7 @@ gemm_kernel(const __grid_constant__ GemmArgs args, int* __restrict__ status) {
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty_bar + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_index();
   const int lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
@@ -538,10 +551,11 @@ gemm_kernel(const __grid_constant__ GemmArgs args, int* __restrict__ status) {
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = warp_uniform(*tmem_slot);
 
   Dims d;
   load_dims<BN>(args, d);
+  make_uniform(d);
   const int total_tiles = d.tiles[0] + d.tiles[1];
 
   if (puller) {
@@ -553,49 +567,44 @@ gemm_kernel(const __grid_constant__ GemmArgs args, int* __restrict__ status) {
     }
   } else if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    // (one elected lane issues, the whole warp runs the loop: addresses and coordinates stay in uniform registers)
+    if (elect_one()) {
       for (int i = 0; i < args.nprob; ++i) {
         tma_prefetch_desc(&args.p[i].tmA);
         tma_prefetch_desc(&args.p[i].tmB);
       }
-      int s = 0;
-      uint32_t phase = 0;
-      bool ok = true;
-      int ag_ready[2] = {0, 0};  // MN-major B: 256-row blocks of the weight known to be in place
-      for (int t = cta; t < total_tiles && ok; t += ncta) {
-        const TileInfo ti = decode_tile(d, t, gathered, rot0, rot1);
-        const Problem& p = args.p[ti.prob];
-        const int m_base = d.m0[ti.prob] + ti.mt * BM;
-        const int n_base = ti.nt * BN;
-        const int k_base = d.k0[ti.prob];
-        const int nkb = (d.K[ti.prob] + BK - 1) / BK;
-        if (!WX_CHK(ti.mt >= 0 && ti.mt < d.tiles_m[ti.prob] && ti.nt >= 0 && ti.nt < d.tiles_n[ti.prob] && (k_base & 7) == 0,
-                    2004, ti.mt, ti.nt)) {
-          *abort_flag = 1;
-          break;
-        }
-        for (int kb = 0; kb < nkb; ++kb) {
-          if (gathered) {
-            if (!B_MN) {
-              if (kb == 0 && !ag_wait(&args.ag[ti.prob].flags[ti.nt], args.ag[ti.prob].target, abort_flag)) {
-                ok = false;
-                break;
-              }
-            } else {
-              const int blk = (k_base + kb * BK + BK - 1) >> 8;
-              if (blk >= ag_ready[ti.prob]) {
-                if (!ag_wait(&args.ag[ti.prob].flags[blk], args.ag[ti.prob].target, abort_flag)) {
-                  ok = false;
-                  break;
-                }
-                ag_ready[ti.prob] = blk + 1;  // pullers finish tiles in order
-              }
+    }
+    int s = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    int ag_ready[2] = {0, 0};  // MN-major B: 256-row blocks of the weight known to be in place
+    for (int t = cta; t < total_tiles && ok; t += ncta) {
+      const TileInfo ti = decode_tile(d, t, gathered, rot0, rot1);
+      const Problem& p = args.p[ti.prob];
+      const int m_base = d.m0[ti.prob] + ti.mt * BM;
+      const int n_base = ti.nt * BN;
+      const int k_base = d.k0[ti.prob];
+      const int nkb = (d.K[ti.prob] + BK - 1) / BK;
+      if (!WX_CHK(ti.mt >= 0 && ti.mt < d.tiles_m[ti.prob] && ti.nt >= 0 && ti.nt < d.tiles_n[ti.prob] && (k_base & 7) == 0,
+                  2004, ti.mt, ti.nt)) {
+        *abort_flag = 1;
+        break;
+      }
+      for (int kb = 0; kb < nkb; ++kb) {
+        if (gathered) {
+          if (!B_MN) {
+            if (kb == 0) ok = ag_wait(&args.ag[ti.prob].flags[ti.nt], args.ag[ti.prob].target, abort_flag);
+          } else {
+            const int blk = (k_base + kb * BK + BK - 1) >> 8;
+            if (blk >= ag_ready[ti.prob]) {
+              ok = ag_wait(&args.ag[ti.prob].flags[blk], args.ag[ti.prob].target, abort_flag);
+              ag_ready[ti.prob] = blk + 1;  // pullers finish tiles in order
             }
           }
-          if (!mbar_wait(&empty_bar[s], phase ^ 1u, abort_flag)) {
-            ok = false;
-            break;
-          }
+        }
+        ok = __all_sync(0xffffffffu, ok && mbar_wait(&empty_bar[s], phase ^ 1u, abort_flag));
+        if (!ok) break;
+        if (elect_one()) {
           uint8_t* sA = smem + s * C::STAGE_BYTES;
           uint8_t* sB = sA + C::A_BYTES;
           mbar_arrive_expect_tx(&full_bar[s], C::STAGE_BYTES);
@@ -612,53 +621,50 @@ gemm_kernel(const __grid_constant__ GemmArgs args, int* __restrict__ status) {
 #pragma unroll
             for (int j = 0; j < BN / 64; ++j) tma_load_2d(sB + j * 8192, &p.tmB, &full_bar[s], n_base + 64 * j, kc);
           }
-          if (++s == C::STAGES) {
-            s = 0;
-            phase ^= 1u;
-          }
+        }
+        if (++s == C::STAGES) {
+          s = 0;
+          phase ^= 1u;
         }
       }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      constexpr uint32_t idesc = make_idesc_bf16(BM, BN, A_MN, B_MN);
-      int s = 0;
-      uint32_t phase = 0;
-      int it = 0;
-      bool ok = true;
-      for (int t = cta; t < total_tiles && ok; t += ncta, ++it) {
-        const TileInfo ti = decode_tile(d, t, gathered, rot0, rot1);
-        const int nkb = (d.K[ti.prob] + BK - 1) / BK;
-        const int acc = it & 1;
-        const uint32_t acc_phase = (it >> 1) & 1;
-        if (!mbar_wait(&tempty_bar[acc], acc_phase ^ 1u, abort_flag)) break;
+    // the whole warp runs the loop and one elected lane issues: the descriptors then live in uniform registers
+    constexpr uint32_t idesc = make_idesc_bf16(BM, BN, A_MN, B_MN);
+    const uint32_t smem_addr = smem_u32(smem);
+    const uint64_t da0 = A_MN ? make_smem_desc_sw128(smem_addr, 8192, 1024) : make_smem_desc_sw128(smem_addr, 16, 1024);
+    const uint64_t db0 = B_MN ? make_smem_desc_sw128(smem_addr + C::A_BYTES, 8192, 1024)
+                              : make_smem_desc_sw128(smem_addr + C::A_BYTES, 16, 1024);
+    constexpr uint32_t a_step = (A_MN ? 2048 : 32) >> 4, b_step = (B_MN ? 2048 : 32) >> 4;  // 16 k
+    int s = 0;
+    uint32_t phase = 0;
+    int it = 0;
+    bool ok = true;
+    for (int t = cta; t < total_tiles && ok; t += ncta, ++it) {
+      const TileInfo ti = decode_tile(d, t, gathered, rot0, rot1);
+      const int nkb = (d.K[ti.prob] + BK - 1) / BK;
+      const int acc = it & 1;
+      const uint32_t acc_phase = (it >> 1) & 1;
+      if (!__all_sync(0xffffffffu, mbar_wait(&tempty_bar[acc], acc_phase ^ 1u, abort_flag))) break;
+      tc_fence_after();
+      const uint32_t tmem_d = tmem_base + acc * BN;
+      for (int kb = 0; kb < nkb; ++kb) {
+        ok = __all_sync(0xffffffffu, mbar_wait(&full_bar[s], phase, abort_flag));
+        if (!ok) break;
         tc_fence_after();
-        const uint32_t tmem_d = tmem_base + acc * BN;
-        for (int kb = 0; kb < nkb; ++kb) {
-          if (!mbar_wait(&full_bar[s], phase, abort_flag)) {
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          const uint32_t a_addr = smem_u32(smem + s * C::STAGE_BYTES);
-          const uint32_t b_addr = a_addr + C::A_BYTES;
+        const uint64_t da = da0 + s * (C::STAGE_BYTES >> 4), db = db0 + s * (C::STAGE_BYTES >> 4);
+        if (elect_one()) {
 #pragma unroll
-          for (int k = 0; k < BK / 16; ++k) {
-            const uint64_t da = A_MN ? make_smem_desc_sw128(a_addr + k * 2048, 8192, 1024)
-                                     : make_smem_desc_sw128(a_addr + k * 32, 16, 1024);
-            const uint64_t db = B_MN ? make_smem_desc_sw128(b_addr + k * 2048, 8192, 1024)
-                                     : make_smem_desc_sw128(b_addr + k * 32, 16, 1024);
-            tc_mma_bf16(tmem_d, da, db, idesc, (kb | k) != 0 ? 1u : 0u);
-          }
+          for (int k = 0; k < BK / 16; ++k) tc_mma_bf16(tmem_d, da + k * a_step, db + k * b_step, idesc, (kb | k) != 0 ? 1u : 0u);
           tc_commit(&empty_bar[s]);
-          if (++s == C::STAGES) {
-            s = 0;
-            phase ^= 1u;
-          }
         }
-        if (ok) tc_commit(&tfull_bar[acc]);
+        if (++s == C::STAGES) {
+          s = 0;
+          phase ^= 1u;
+        }
       }
+      if (ok && elect_one()) tc_commit(&tfull_bar[acc]);
     }
   } else {
     // ------------------------------------------------------------------ epilogue

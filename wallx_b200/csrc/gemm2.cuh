@@ -53,7 +53,7 @@ gemm_pair_kernel(const __grid_constant__ GemmArgs args, int* __restrict__ status
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty_bar + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_index();
   const int lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
   const bool leader = rank == 0;
@@ -83,10 +83,11 @@ gemm_pair_kernel(const __grid_constant__ GemmArgs args, int* __restrict__ status
   cluster_arrive();  // barriers and tensor memory of both CTAs exist before anything crosses
   cluster_wait();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = warp_uniform(*tmem_slot);
 
   Dims d;
   load_dims<kPairTileN, kPairTileM>(args, d);
+  make_uniform(d);
   const int total_tiles = d.tiles[0] + d.tiles[1];
   const int pair = (static_cast<int>(blockIdx.x) - n_pull) >> 1;
   const int npair = (static_cast<int>(gridDim.x) - n_pull) >> 1;
@@ -100,48 +101,44 @@ gemm_pair_kernel(const __grid_constant__ GemmArgs args, int* __restrict__ status
     }
   } else if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer (both CTAs)
-    if (lane == 0) {
+    // (one elected lane issues, the whole warp runs the loop: addresses and coordinates stay in uniform registers)
+    if (elect_one()) {
       for (int i = 0; i < args.nprob; ++i) {
         tma_prefetch_desc(&args.p[i].tmA);
         tma_prefetch_desc(&args.p[i].tmB);
       }
-      int s = 0;
-      uint32_t phase = 0;
-      bool ok = true;
-      int ag_ready[2] = {0, 0};  // MN-major B: 256-row blocks of the weight known to be in place
-      for (int t = pair; t < total_tiles && ok; t += npair) {
-        const TileInfo ti = decode_tile(d, t, gathered, rot0, rot1);
-        const Problem& p = args.p[ti.prob];
-        const int m_base = d.m0[ti.prob] + ti.mt * kPairTileM + static_cast<int>(rank) * BM;
-        const int n_base = ti.nt * kPairTileN + static_cast<int>(rank) * 128;
-        const int k_base = d.k0[ti.prob];
-        const int nkb = (d.K[ti.prob] + BK - 1) / BK;
-        for (int kb = 0; kb < nkb; ++kb) {
-          if (gathered) {
-            if (!B_MN) {  // the pair's 256 weight rows are one flag tile
-              if (kb == 0 && !ag_wait(&args.ag[ti.prob].flags[ti.nt], args.ag[ti.prob].target, abort_flag)) {
-                ok = false;
-                break;
-              }
-            } else {
-              const int blk = (k_base + kb * BK + BK - 1) >> 8;
-              if (blk >= ag_ready[ti.prob]) {
-                if (!ag_wait(&args.ag[ti.prob].flags[blk], args.ag[ti.prob].target, abort_flag)) {
-                  ok = false;
-                  break;
-                }
-                ag_ready[ti.prob] = blk + 1;  // pullers finish tiles in order
-              }
+    }
+    const uint32_t full_leader = mapa_u32(smem_u32(full_bar), 0);
+    int s = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    int ag_ready[2] = {0, 0};  // MN-major B: 256-row blocks of the weight known to be in place
+    for (int t = pair; t < total_tiles && ok; t += npair) {
+      const TileInfo ti = decode_tile(d, t, gathered, rot0, rot1);
+      const Problem& p = args.p[ti.prob];
+      const int m_base = d.m0[ti.prob] + ti.mt * kPairTileM + static_cast<int>(rank) * BM;
+      const int n_base = ti.nt * kPairTileN + static_cast<int>(rank) * 128;
+      const int k_base = d.k0[ti.prob];
+      const int nkb = (d.K[ti.prob] + BK - 1) / BK;
+      for (int kb = 0; kb < nkb; ++kb) {
+        if (gathered) {
+          if (!B_MN) {  // the pair's 256 weight rows are one flag tile
+            if (kb == 0) ok = ag_wait(&args.ag[ti.prob].flags[ti.nt], args.ag[ti.prob].target, abort_flag);
+          } else {
+            const int blk = (k_base + kb * BK + BK - 1) >> 8;
+            if (blk >= ag_ready[ti.prob]) {
+              ok = ag_wait(&args.ag[ti.prob].flags[blk], args.ag[ti.prob].target, abort_flag);
+              ag_ready[ti.prob] = blk + 1;  // pullers finish tiles in order
             }
           }
-          if (!mbar_wait(&empty_bar[s], phase ^ 1u, abort_flag)) {
-            ok = false;
-            break;
-          }
+        }
+        ok = __all_sync(0xffffffffu, ok && mbar_wait(&empty_bar[s], phase ^ 1u, abort_flag));
+        if (!ok) break;
+        if (elect_one()) {
           uint8_t* sA = smem + s * kPairStageBytes;
           uint8_t* sB = sA + kPairABytes;
           if (leader) mbar_arrive_expect_tx(&full_bar[s], 2 * kPairStageBytes);
-          const uint32_t full0 = mapa_u32(smem_u32(&full_bar[s]), 0);
+          const uint32_t full0 = full_leader + s * 8;
           const int kc = k_base + kb * BK;
           if (!A_MN) {
             tma_load_2d_pair(sA, &p.tmA, full0, kc, m_base);
@@ -155,17 +152,25 @@ gemm_pair_kernel(const __grid_constant__ GemmArgs args, int* __restrict__ status
 #pragma unroll
             for (int j = 0; j < 2; ++j) tma_load_2d_pair(sB + j * 8192, &p.tmB, full0, n_base + 64 * j, kc);
           }
-          if (++s == kPairStages) {
-            s = 0;
-            phase ^= 1u;
-          }
+        }
+        if (++s == kPairStages) {
+          s = 0;
+          phase ^= 1u;
         }
       }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer (leader only)
-    if (lane == 0 && leader) {
+    if (leader) {
+      // the whole warp runs the loop and one elected lane issues: the descriptors then live in uniform registers
       constexpr uint32_t idesc = make_idesc_bf16(kPairTileM, kPairTileN, A_MN, B_MN);
+      const uint32_t smem_addr = smem_u32(smem);
+      const uint64_t da0 = A_MN ? make_smem_desc_sw128(smem_addr, 8192, 1024) : make_smem_desc_sw128(smem_addr, 16, 1024);
+      const uint64_t db0 = B_MN ? make_smem_desc_sw128(smem_addr + kPairABytes, 8192, 1024)
+                                : make_smem_desc_sw128(smem_addr + kPairABytes, 16, 1024);
+      constexpr uint32_t a_step = (A_MN ? 2048 : 32) >> 4, b_step = (B_MN ? 2048 : 32) >> 4;  // 16 k
+      const uint32_t empty0 = smem_u32(empty_bar), empty1 = mapa_u32(empty0, 1);
+      const uint32_t tfull0 = smem_u32(tfull_bar), tfull1 = mapa_u32(tfull0, 1);
       int s = 0;
       uint32_t phase = 0;
       int it = 0;
@@ -175,38 +180,30 @@ gemm_pair_kernel(const __grid_constant__ GemmArgs args, int* __restrict__ status
         const int nkb = (d.K[ti.prob] + BK - 1) / BK;
         const int acc = it & 1;
         const uint32_t acc_phase = (it >> 1) & 1;
-        if (!mbar_wait(&tempty_bar[acc], acc_phase ^ 1u, abort_flag)) break;
+        if (!__all_sync(0xffffffffu, mbar_wait(&tempty_bar[acc], acc_phase ^ 1u, abort_flag))) break;
         tc_fence_after();
         const uint32_t tmem_d = tmem_base + acc * kPairTileN;
         for (int kb = 0; kb < nkb; ++kb) {
-          if (!mbar_wait(&full_bar[s], phase, abort_flag)) {
-            ok = false;
-            break;
-          }
+          ok = __all_sync(0xffffffffu, mbar_wait(&full_bar[s], phase, abort_flag));
+          if (!ok) break;
           tc_fence_after();
-          const uint32_t a_addr = smem_u32(smem + s * kPairStageBytes);
-          const uint32_t b_addr = a_addr + kPairABytes;
+          const uint64_t da = da0 + s * (kPairStageBytes >> 4), db = db0 + s * (kPairStageBytes >> 4);
+          if (elect_one()) {
 #pragma unroll
-          for (int k = 0; k < BK / 16; ++k) {
-            const uint64_t da = A_MN ? make_smem_desc_sw128(a_addr + k * 2048, 8192, 1024)
-                                     : make_smem_desc_sw128(a_addr + k * 32, 16, 1024);
-            const uint64_t db = B_MN ? make_smem_desc_sw128(b_addr + k * 2048, 8192, 1024)
-                                     : make_smem_desc_sw128(b_addr + k * 32, 16, 1024);
-            tc_mma_bf16_pair(tmem_d, da, db, idesc, (kb | k) != 0 ? 1u : 0u);
+            for (int k = 0; k < BK / 16; ++k)
+              tc_mma_bf16_pair(tmem_d, da + k * a_step, db + k * b_step, idesc, (kb | k) != 0 ? 1u : 0u);
+            // the stage is free in both CTAs once these MMAs have read it
+            tc_commit_pair(empty0 + s * 8);
+            tc_commit_pair(empty1 + s * 8);
           }
-          // the stage is free in both CTAs once these MMAs have read it
-          const uint32_t e = smem_u32(&empty_bar[s]);
-          tc_commit_pair(e);
-          tc_commit_pair(mapa_u32(e, 1));
           if (++s == kPairStages) {
             s = 0;
             phase ^= 1u;
           }
         }
-        if (ok) {
-          const uint32_t f = smem_u32(&tfull_bar[acc]);
-          tc_commit_pair(f);
-          tc_commit_pair(mapa_u32(f, 1));
+        if (ok && elect_one()) {
+          tc_commit_pair(tfull0 + acc * 8);
+          tc_commit_pair(tfull1 + acc * 8);
         }
       }
     }

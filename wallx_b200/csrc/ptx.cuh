@@ -41,6 +41,16 @@ __device__ __forceinline__ bool elect_one() {
   return pred != 0;
 }
 
+// Values that the compiler knows to be the same in all lanes. The warps that issue TMA loads and tcgen05.mma run their
+// loops converged (all lanes wait, one elected lane issues) on such values: addresses, descriptors and coordinates then
+// live in uniform registers, where those instructions take their operands from. With the loop inside `if (lane == 0)`
+// every descriptor was computed in the lane's registers and moved over, about 0.1 us per 64-wide k step, and that thread
+// bounded all kernels: 8192 x 4096 x 4096 on CTA pairs 191 -> 181 us, 128-wide tiles 328 -> 238, packed causal attention
+// of 32 x 346 tokens forward 133 -> 83 and backward 534 -> 332.
+__device__ __forceinline__ int warp_uniform(int x) { return __shfl_sync(0xffffffffu, x, 0); }
+__device__ __forceinline__ uint32_t warp_uniform(uint32_t x) { return __shfl_sync(0xffffffffu, x, 0); }
+__device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0); }
+
 // ----------------------------------------------------------------------------- mbarrier
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
