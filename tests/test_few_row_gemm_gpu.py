@@ -1,0 +1,79 @@
+"""Few-row GEMM (csrc/gemm_skinny.cuh): tile, split and epilogue edges against fp32."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _rand(g, *shape, scale=1.0):
+    return (torch.randn(*shape, generator=g) * scale).to(torch.bfloat16).cuda()
+
+
+def _check(got, want, K, what):
+    # the stored value is rounded to bf16 (2^-9 of itself) and an fp32 sum of K products carries at most K * 2^-24 of the
+    # sum of their magnitudes, here below 2^-9 of the largest result
+    err = (got.float() - want.float()).abs().max().item()
+    bound = (2.0 ** -8 + K * 2.0 ** -22) * want.float().abs().max().item()
+    assert err <= bound, f"{what}: {err} > {bound}"
+
+
+def _gemm(G, spec, M):
+    if M <= 128:
+        G.launch([spec], force_bn=16)
+    else:
+        with torch.no_grad(), G.inference_kernels():
+            G.launch([spec])
+
+
+@pytest.mark.parametrize("M", [1, 15, 16, 17, 64, 65, 128, 129, 155, 256, 257, 314, 1000])
+@pytest.mark.parametrize("N,K", [(20, 64), (100, 200), (129, 2048), (2080, 2048), (512, 8192)])
+def test_bias_residual_rows_and_columns_at_tile_edges(M, N, K):
+    from wallx_b200.ops import gemm as G
+
+    g = torch.Generator().manual_seed(M + N + K)
+    a, w = _rand(g, M, K), _rand(g, N, K, scale=0.05)
+    bias, res = _rand(g, N), _rand(g, M, N)
+    out = torch.full((M + 1, N), 7.0, device="cuda", dtype=torch.bfloat16)
+    _gemm(G, G.GemmSpec(a, w, out[:M], bias=bias, residual=res), M)
+    torch.cuda.synchronize()
+    G.check_status()
+    _check(out[:M], a.float() @ w.float().t() + bias.float() + res.float(), K, "bias + residual")
+    assert bool((out[M] == 7.0).all()), "wrote past the last row"
+
+
+@pytest.mark.parametrize("M", [3, 32, 70, 200])
+def test_epilogues(M):
+    from wallx_b200.ops import gemm as G
+    from wallx_b200.ops import ref
+
+    g = torch.Generator().manual_seed(M)
+    K, I = 4096, 160
+    a, w = _rand(g, M, K), _rand(g, 2 * I, K, scale=0.02)
+    full = a.float() @ w.float().t()
+    # fp32 output that is added to
+    acc = torch.randn(M, 2 * I, generator=g).cuda()
+    want = acc + full
+    _gemm(G, G.GemmSpec(a, w, acc, flags=G.OUT_FP32 | G.ACCUMULATE), M)
+    _check(acc, want, K, "fp32 accumulate")
+    # SwiGLU with the raw gate / up values kept
+    h, raw = torch.empty(M, I, device="cuda", dtype=torch.bfloat16), torch.empty(M, 2 * I, device="cuda", dtype=torch.bfloat16)
+    _gemm(G, G.GemmSpec(a, w, h, out2=raw, flags=G.ACT_SWIGLU), M)
+    _check(raw, full, K, "raw gate / up")
+    _check(h, ref.swiglu_interleaved(raw.float()), K, "SwiGLU")
+    # GELU, rows scattered through a map with one row dropped
+    out = torch.zeros(M + 5, 2 * I, device="cuda", dtype=torch.bfloat16)
+    row_map = torch.randperm(M + 5, generator=g)[:M].to(torch.int32)
+    row_map[0] = -1
+    _gemm(G, G.GemmSpec(a, w, out, row_map=row_map.cuda(), flags=G.ACT_GELU), M)
+    want = torch.zeros(M + 5, 2 * I, device="cuda")
+    want[row_map[1:].long().cuda()] = torch.nn.functional.gelu(full[1:])
+    _check(out, want, K, "GELU + row map")
+    if M <= 128:  # SwiGLU backward: the accumulator is dL/dh of 2 * I channels
+        gu = _rand(g, M, 4 * I)
+        dgu = torch.empty_like(gu)
+        G.launch([G.GemmSpec(a, w, dgu, out2=gu, flags=G.SWIGLU_BWD)], force_bn=16)
+        wide = torch.empty_like(gu)
+        G.launch([G.GemmSpec(a, w, wide, out2=gu, flags=G.SWIGLU_BWD)], force_bn=64)
+        _check(dgu, wide, K, "SwiGLU backward")
+    torch.cuda.synchronize()
+    G.check_status()

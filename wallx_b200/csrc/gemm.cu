@@ -857,7 +857,7 @@ namespace wx {
 
 namespace {
 // TFLOP/s of the 128 x {256, 128, 64} single-CTA tiles and of the 256 x 256 CTA-pair tile on a large problem.
-double g_tile_rates[4] = {1260.0, 970.0, 525.0, 1360.0};
+double g_tile_rates[4] = {1430.0, 1155.0, 705.0, 1540.0};
 }  // namespace
 
 void gemm_set_tile_rates(const double* rates4) {
@@ -874,52 +874,62 @@ int gemm_launch(const GemmCall* calls, int ncalls, cudaStream_t stream, int* sta
   for (int i = 1; i < ncalls; ++i)
     if (calls[i].a_mn != a_mn || calls[i].b_mn != b_mn) return -2;
 
-  // Few rows (decode, denoise steps): clusters of CTAs that split K (gemm_skinny.cuh). force_bn = 16 selects that
-  // kernel where it is legal, 17 the same with one CTA per column tile (no split); other forced widths bypass it.
-  // force_bn = 18 is "automatic, inference": it also lets problems of up to 1024 rows whose 128 x 256 tiles fill less
-  // than half of the SMs and whose K is 4096 or more run on K-splitting clusters (prefix passes: few tiles, long K, one
-  // serial chain per tile).
-  // Training launches (0) take neither that second path nor a K split of the few-row kernel, so a different summation
-  // order cannot enter a comparison of training runs.
+  // Few rows: the kernel of gemm_skinny.cuh. force_bn = 16 selects it where it is legal, 17 the same with one CTA per tile
+  // (no split of K); other forced widths bypass it. force_bn = 18 is "automatic, inference". Training launches (0) never
+  // split K, so a different summation order cannot enter a comparison of training runs (the fused-gather GEMM of a
+  // row-sharded weight is the general kernel, and the plans are compared bit for bit).
   const bool infer = force_bn == 18;
   if (infer) force_bn = 0;
   if (!a_mn && !b_mn && (force_bn == 0 || force_bn == 16 || force_bn == 17)) {
-    int max_m = 0, min_nkb = 1 << 30;
-    long st = 0, mid = 0;
+    int max_m = 0, min_nkb = 1 << 30, max_nkb = 0;
     bool plain = true;
+    long tiles = 0;
     for (int i = 0; i < ncalls; ++i) {
       max_m = calls[i].M > max_m ? calls[i].M : max_m;
-      st += (calls[i].N + kSkinnyBN - 1) / kSkinnyBN;
-      mid += static_cast<long>((calls[i].N + kMidBN - 1) / kMidBN) * ((calls[i].M + BM - 1) / BM);
       const int nkb = (calls[i].K + BK - 1) / BK;
       min_nkb = nkb < min_nkb ? nkb : min_nkb;
+      max_nkb = nkb > max_nkb ? nkb : max_nkb;
+      tiles += (calls[i].N + kFewBN - 1) / kFewBN;
       if ((calls[i].flags & (GEMM_ACT_SWIGLU | GEMM_SWIGLU_BWD)) && (calls[i].N % 32 != 0)) plain = false;
       if (calls[i].flags & GEMM_ZERO_PAD_ROWS) plain = false;  // rows past M are never visited by that kernel
     }
-    if (plain && max_m >= 1 && max_m <= BM && st >= 1 && st <= 1024) {
-      GemmArgs sargs;
-      const int a_rows = skinny_rows(max_m);
-      const int src = fill_args(sargs, calls, ncalls, kSkinnyBN, a_rows);
-      if (src != 0) return src;
-      // K is split over a cluster for inference launches only: a training launch must give the bits of the general
-      // kernel (the fused-gather GEMM of a row-sharded weight is that kernel, and the plans are compared bit for bit)
-      const int splits = (infer || force_bn == 16) ? skinny_splits(st, min_nkb, num_sms()) : 1;
-      return launch_skinny(sargs, a_rows, kSkinnyBN, static_cast<int>(st), splits, stream, status);
+    plain = plain && max_m >= 1 && tiles >= 1;
+    if (plain && max_m <= BM && (infer || force_bn == 16)) {
+      const FewShape sh = few_shape(max_m, tiles, min_nkb);
+      const int rc = launch_few(calls, ncalls, sh, stream, status);
+      if (rc != -12) return rc;
+    }
+    // Without a split a CTA walks all of K: worth it where the weight slices alone fill the device (22016 x 2048, 62 rows:
+    // 25 against 35 us), not for a narrow one (2048 x 2048, 62 rows: 14.8 against 11.4 us for 64-wide tiles).
+    if (plain && max_m <= BM && (force_bn == 17 || (force_bn == 0 && !infer && max_m <= 64 && tiles >= num_sms()))) {
+      FewShape sh = few_shape(max_m, tiles, min_nkb);
+      sh.splits = 1;
+      const int rc = launch_few(calls, ncalls, sh, stream, status);
+      if (rc != -12) return rc;
     }
     if (force_bn == 16 || force_bn == 17) return -11;
-    // (measured in CUDA graphs at 314 rows: 35 against 54 us for K = 11008, but 24 against 15 us for K = 2048, where the
-    // hand-over and reduction of 128 x 256 partial tiles costs more than the shorter chain saves: long K only)
-    static const int mid_min_nkb = [] {
-      const char* e = getenv("WX_MID_MIN_NKB");
-      return e ? atoi(e) : 64;
-    }();
-    if (infer && plain && max_m > BM && max_m <= 1024 && mid >= 1 && min_nkb >= mid_min_nkb) {
-      const int splits = skinny_splits(mid, min_nkb, num_sms());
-      if (splits >= 2) {
-        GemmArgs sargs;
-        const int src = fill_args(sargs, calls, ncalls, kMidBN, BM);
-        if (src != 0) return src;
-        return launch_skinny(sargs, BM, kMidBN, static_cast<int>(mid), splits, stream, status);
+    if (infer && plain && max_m > BM && max_m <= 1024) {
+      // A few hundred rows (prefix passes, denoise steps of several sequences): the weight slices split along K, or the
+      // general kernel, whose tiles are one serial chain of k steps each. Microseconds, fitted to 8 shapes x 8 row counts
+      // (155 rows, 2048 x 2048: 10.6 against 11.7; 314 rows, K = 11008: 21 against 41; 256 rows, K = 2048: 13.2 against
+      // 11.3); the margin leaves near ties to the general kernel.
+      const FewShape sh = few_shape(max_m, tiles, min_nkb);
+      const long few_tiles = tiles * ((max_m + sh.nb - 1) / sh.nb);
+      const int cap = few_capacity(sh);
+      const double few = 5.4 + 0.023 * sh.nb + (max_nkb + sh.splits - 1) / sh.splits * (sh.nb <= 160 ? 0.21 : 0.32);
+      const int widths[3] = {64, 128, 256};
+      const double step[3] = {0.19, 0.22, 0.36};
+      double chain = 1e30;
+      for (int w = 0; w < 3; ++w) {
+        long t = 0;
+        for (int i = 0; i < ncalls; ++i)
+          t += static_cast<long>((calls[i].M + BM - 1) / BM) * ((calls[i].N + widths[w] - 1) / widths[w]);
+        const double c = static_cast<double>((t + num_sms() - 1) / num_sms()) * step[w];
+        chain = c < chain ? c : chain;
+      }
+      if (few_tiles <= cap && few < 0.92 * (5.5 + max_nkb * chain)) {
+        const int rc = launch_few(calls, ncalls, sh, stream, status);
+        if (rc != -12) return rc;
       }
     }
   }

@@ -1,90 +1,196 @@
-// Few-row GEMM for sm_100a: out[M <= 128, N] = A[M, K] . W[N, K]^T, both operands K-major (decode and denoise steps:
-// 32 action rows against every weight of a layer). Included by gemm.cu after the general kernel.
+// Few-row GEMM for sm_100a: out[M, N] = A[M, K] . W[N, K]^T, both operands K-major (decoding and denoise steps: a handful
+// to a few hundred activation rows against every weight of a layer). Included by gemm.cu after the general kernel.
 //
-// What limits such a product is neither the tensor pipe nor DRAM but the serial chain inside one CTA: measured on a
-// B200, a CTA of the general kernel (or of a one-CTA-per-column-tile variant of it) spends about 0.3 us per 64-wide
-// k block (wait for the stage, four tcgen05.mma whose 128-row A operand is read from shared memory whatever the row
-// count, commit), i.e. 10 us for K = 2048 with every unit of the GPU idle. So the work is cut along K as well:
-//   * one *cluster* of `splits` CTAs per 64 output columns, CTA r of the cluster owning the k blocks
-//     [nkb * r / splits, nkb * (r + 1) / splits) -- 2048 x 2048 runs as 32 clusters of 4, eight k blocks per CTA;
-//   * a stage holds only the rows that exist (32, 64 or 128) and a 64-row slice of the weight; with so few k blocks
-//     per CTA all of its loads are in flight at once and a stage is handed back only if the ring actually wraps;
-//   * every CTA leaves its fp32 partial tile in its own shared memory; after a cluster barrier the (row, 32-column)
-//     pieces of the tile are dealt round-robin to the threads of all CTAs of the cluster, which add the partials in
-//     rank order through distributed shared memory (a fixed order: results do not depend on timing) and run the
-//     usual epilogue (bias / SwiGLU / residual / fp32 / accumulate / row map).
-// tcgen05.mma runs at M = 128 whatever the row count: the A descriptor reaches past the loaded rows into the bytes
-// that follow in shared memory (the B slice, later stages, a slack area after the last stage). Those accumulator
-// rows hold garbage, stay in their own TMEM lanes and are never stored. With one split the sum over K has the order
-// of the general kernel (bit-identical results); with more it is a sum of per-split partial sums.
+// Such a product reads far more weight than anything else, and what limits it is the time one SM needs for its share:
+//   * the roles of the operands are swapped. The 128 rows of the MMA are output columns (a slice of the weight) and the
+//     activation rows are its N, so a 64-wide k step stages 16 KB of weight and `nb` x 128 bytes of activations and the
+//     tensor core reads exactly that. (With the activations as the 128-row operand, 32 rows cost as much as 128 and a
+//     weight slice of 64 rows cost 0.1 us per k step whatever arrived.)
+//   * one *cluster* of `splits` CTAs per 128 output columns, CTA r of the cluster owning the k blocks
+//     [nkb * r / splits, nkb * (r + 1) / splits): 2048 x 2048 runs as 16 clusters of 8, four k blocks per CTA.
+//   * every CTA leaves its fp32 partial tile in its own shared memory as rows of 128 output columns; after a cluster
+//     barrier the rows are dealt to the warps of the cluster, which add the partials in rank order through distributed
+//     shared memory (a fixed order: results do not depend on timing), a whole 512-byte row per load, and run the epilogue
+//     on four columns per lane, so every global access is a contiguous row as well.
+// With one split the sum over K has the order of the general kernel (bit-identical results); with more it is a sum of
+// per-split partial sums.
+//
+// Measured (B200, us per call in a CUDA graph that reads other weights each time, before -> now; last column: now as
+// dependent launches):
+//   32 x 2048 x 2048 (rows, columns, K)   10.8 -> 8.0    5.9
+//   1 x 2048 x 11008                      14.8 -> 13.4  12.3   (6.8 us of weight bytes)
+//   1 x 22016 x 2048 SwiGLU               30.5 -> 19.4  18.1   (13.6 us of weight bytes)
+//   6 x 153986 x 2048                      135 -> 98          (95 us of weight bytes)
+//   155 x 2048 x 2048                     14.5 -> 10.8
+//   314 x 2048 x 11008                      38 -> 21
+// Short products are left with the latency of a launch, the first loads, the cluster barriers and the reduction; the long
+// ones stand at 75 to 97 % of the copy bandwidth.
 #pragma once
+
+#include <atomic>
 
 namespace wx {
 namespace {
 
-constexpr int kSkinnyBN = 64;
-constexpr int kSkinnyThreads = 192;  // TMA warp, MMA warp, 4 epilogue warps (one per TMEM lane quarter)
-constexpr int kMidBN = 256;    // tile width of the same kernel for 129..1024 rows (128-row tiles, see gemm_launch)
-constexpr int kSkinnyMaxSplits = 8;          // portable cluster size
+constexpr int kFewBN = 128;            // output columns per tile (rows of the weight slice)
+constexpr int kFewThreads = 320;       // TMA warp, MMA warp, 8 warps that move the accumulator (two per TMEM lane quarter)
+constexpr int kFewWarps = kFewThreads / 32;
+constexpr int kFewMaxRows = 256;       // activation rows per tile: the N of an MMA
+constexpr int kFewMaxSplits = 8;       // portable cluster size
+constexpr int kFewBBytes = kFewBN * BK * 2;
+
+struct FewShape {
+  int nb;      // activation rows per tile: a multiple of 16
+  int stages;
+  int splits;
+};
 
 __device__ __forceinline__ void prefetch_l1(const void* p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
 
-template <int A_ROWS, int BN>
-struct SkinnyCfg {
-  static constexpr int A_BYTES = A_ROWS * BK * 2;
-  static constexpr int PITCH = BN + 4;  // floats per row of the partial tile (16-byte row stores without conflicts)
-  static constexpr int B_BYTES = BN * BK * 2;
-  static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-  // about 100 KB of stages, so that two CTAs fit on an SM: under programmatic dependent launch the CTAs of the next
-  // few-row GEMM then sit beside this one's and stream their weights while this one finishes
-  static constexpr int STAGES = (BN == 256) ? 4 : (A_ROWS == 32) ? 8 : (A_ROWS == 64) ? 6 : 4;
-  static constexpr int SLACK = BM * BK * 2 - A_BYTES;  // what the 128-row A descriptor reads beyond the last stage's rows
-  static constexpr int PARTIAL_BYTES = A_ROWS * PITCH * 4;  // aliases the start of the ring once the MMAs are done
-  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + SLACK + 1024 + 512;
-  static_assert(SMEM_BYTES <= 227 * 1024, "stage ring does not fit");
-  static_assert(STAGE_BYTES % 1024 == 0, "stages must keep the 1024-byte alignment of the swizzle pattern");
-  static_assert(PARTIAL_BYTES <= STAGES * STAGE_BYTES, "partial tile must fit in the ring");
-};
+__device__ __forceinline__ float4 bf16x4_to_f32(uint2 x) {
+  const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&x.x));
+  const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&x.y));
+  return make_float4(a.x, a.y, b.x, b.y);
+}
 
-template <int A_ROWS, int BN>
-__global__ void __launch_bounds__(kSkinnyThreads, 1)
-gemm_skinny_kernel(const __grid_constant__ GemmArgs args, int* __restrict__ status, int splits) {
-  using C = SkinnyCfg<A_ROWS, BN>;
-  // Clusters are laid out from the static sizes (problem 0's column tiles, then problem 1's); the row count and K
-  // may be smaller on the device (dyn). Everything that decides whether a CTA works is uniform over its cluster.
+// Epilogue of four consecutive columns [n, n + 4) of destination row `drow`; the lanes of a warp hold 128 consecutive
+// columns of one row. Same arithmetic and order as epilogue_chunk.
+__device__ __forceinline__ void epilogue_quad(const Problem& p, float4 acc, long drow, int n) {
+  const int flags = p.flags;
+  const int nvalid = p.N - n;  // may be zero or negative: such lanes only take part in the exchange
+  float v[4] = {acc.x, acc.y, acc.z, acc.w};
+  if (p.bias != nullptr) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (j < nvalid) v[j] += __bfloat162float(p.bias[n + j]);
+  }
+  if (flags & GEMM_SWIGLU_BWD) {  // v = dL/dh of channels [n, n + 4); N is a multiple of 32
+    if (nvalid <= 0) return;
+    const long off = 2L * (n & ~15) + (n & 15);
+    const __nv_bfloat16* gsrc = reinterpret_cast<const __nv_bfloat16*>(p.D2) + drow * p.ldd2 + off;
+    __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(p.D) + drow * p.ldd + off;
+    const float4 g4 = bf16x4_to_f32(*reinterpret_cast<const uint2*>(gsrc));
+    const float4 u4 = bf16x4_to_f32(*reinterpret_cast<const uint2*>(gsrc + 16));
+    const float g[4] = {g4.x, g4.y, g4.z, g4.w}, u[4] = {u4.x, u4.y, u4.z, u4.w};
+    float dg[4], du[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float s = 1.0f / (1.0f + __expf(-g[j]));
+      dg[j] = v[j] * u[j] * s * (1.0f + g[j] * (1.0f - s));
+      du[j] = v[j] * g[j] * s;
+    }
+    *reinterpret_cast<uint2*>(dst) = make_uint2(pack_bf16x2(dg[0], dg[1]), pack_bf16x2(dg[2], dg[3]));
+    *reinterpret_cast<uint2*>(dst + 16) = make_uint2(pack_bf16x2(du[0], du[1]), pack_bf16x2(du[2], du[3]));
+    return;
+  }
+  if (flags & GEMM_ACT_SWIGLU) {  // blocks of [16 gate | 16 up] columns: lanes 0..3 of eight hold gate, 4..7 up
+    const uint2 raw = make_uint2(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]));
+    if (p.D2 != nullptr && nvalid > 0)
+      *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(p.D2) + drow * p.ldd2 + n) = raw;
+    uint2 up;
+    up.x = __shfl_down_sync(0xffffffffu, raw.x, 4);
+    up.y = __shfl_down_sync(0xffffffffu, raw.y, 4);
+    if (nvalid > 0 && (n & 16) == 0) {  // (gate and up rounded to bf16 first, as in the unfused path)
+      const float4 g = bf16x4_to_f32(raw), u = bf16x4_to_f32(up);
+      *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(p.D) + drow * p.ldd + ((n & ~31) >> 1) + (n & 15)) =
+          make_uint2(pack_bf16x2(silu_f(g.x) * u.x, silu_f(g.y) * u.y), pack_bf16x2(silu_f(g.z) * u.z, silu_f(g.w) * u.w));
+    }
+    return;
+  }
+  if (nvalid <= 0) return;
+  if (flags & GEMM_ACT_GELU) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) v[j] = gelu_erf(v[j]);
+  }
+  if (p.residual != nullptr) {
+    const __nv_bfloat16* rs = p.residual + drow * p.ldr + n;
+    if (nvalid >= 4 && (p.ldr & 3) == 0 && (reinterpret_cast<uintptr_t>(p.residual) & 7) == 0) {
+      const float4 f = bf16x4_to_f32(*reinterpret_cast<const uint2*>(rs));
+      v[0] += f.x;
+      v[1] += f.y;
+      v[2] += f.z;
+      v[3] += f.w;
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (j < nvalid) v[j] += __bfloat162float(rs[j]);
+    }
+  }
+  const bool accum = (flags & GEMM_ACCUMULATE) != 0;
+  if (flags & GEMM_OUT_FP32) {
+    float* dst = reinterpret_cast<float*>(p.D) + drow * p.ldd + n;
+    if (nvalid >= 4 && (p.ldd & 3) == 0 && (reinterpret_cast<uintptr_t>(p.D) & 15) == 0) {
+      float4 o = make_float4(v[0], v[1], v[2], v[3]);
+      if (accum) {
+        const float4 old = *reinterpret_cast<const float4*>(dst);
+        o.x += old.x;
+        o.y += old.y;
+        o.z += old.z;
+        o.w += old.w;
+      }
+      *reinterpret_cast<float4*>(dst) = o;
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (j < nvalid) dst[j] = accum ? dst[j] + v[j] : v[j];
+    }
+  } else {
+    __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(p.D) + drow * p.ldd + n;
+    if (nvalid >= 4 && (p.ldd & 3) == 0 && (reinterpret_cast<uintptr_t>(p.D) & 7) == 0) {
+      if (accum) {
+        const float4 f = bf16x4_to_f32(*reinterpret_cast<const uint2*>(dst));
+        v[0] += f.x;
+        v[1] += f.y;
+        v[2] += f.z;
+        v[3] += f.w;
+      }
+      *reinterpret_cast<uint2*>(dst) = make_uint2(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]));
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (j < nvalid) dst[j] = __float2bfloat16(accum ? __bfloat162float(dst[j]) + v[j] : v[j]);
+    }
+  }
+}
+
+__global__ void __launch_bounds__(kFewThreads, 2)
+gemm_few_kernel(const __grid_constant__ GemmArgs args, int* __restrict__ status, const FewShape sh) {
+  // Clusters are laid out from the static sizes (problem 0's tiles, then problem 1's); the row count and K may be
+  // smaller on the device (dyn). Everything that decides whether a CTA works is uniform over its cluster.
+  const int splits = sh.splits, nb = sh.nb, stages = sh.stages;
   const int tile = static_cast<int>(blockIdx.x) / splits;
   const int rank = static_cast<int>(blockIdx.x) - tile * splits;  // = %cluster_ctarank
-  // tiles of a problem: column tiles x 128-row tiles (static row count), row tiles fastest so that the clusters
-  // which share a weight slice run at the same time
-  const int mt0 = (args.p[0].M + BM - 1) / BM;
-  const int t0 = ((args.p[0].N + BN - 1) / BN) * mt0;
+  // row tiles fastest, so that the clusters which share a weight slice run at the same time
+  const int mt0 = (args.p[0].M + nb - 1) / nb;
+  const int t0 = ((args.p[0].N + kFewBN - 1) / kFewBN) * mt0;
   const int prob = tile < t0 ? 0 : 1;
-  const int mtiles = prob ? (args.p[1].M + BM - 1) / BM : mt0;
+  const int mtiles = prob ? (args.p[1].M + nb - 1) / nb : mt0;
   const int tp = tile - (prob ? t0 : 0);
   const int nt = tp / mtiles;
   const int mt = tp - nt * mtiles;
   if (prob >= args.nprob) return;  // cannot happen with the host's grid
   const Problem& p = args.p[prob];
+  const int stage_bytes = kFewBBytes + nb * (BK * 2);
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + C::STAGES * C::STAGE_BYTES + C::SLACK);
-  uint64_t* empty_bar = full_bar + C::STAGES;
-  uint64_t* tfull_bar = empty_bar + C::STAGES;
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + stages * stage_bytes);
+  uint64_t* empty_bar = full_bar + stages;
+  uint64_t* tfull_bar = empty_bar + stages;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tfull_bar + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  float* partial = reinterpret_cast<float*>(smem);
+  float* partial = reinterpret_cast<float*>(smem);  // [nb][128], over the first stages once the MMAs are done
 
   // ---- prologue: nothing here reads memory that an earlier kernel writes, so under programmatic dependent launch it
-  // runs while the kernel ahead in the stream is still finishing
-  const int warp = threadIdx.x >> 5;
+  // runs while the kernel ahead in the stream is still finishing. With static sizes (no device-side row count or K) the
+  // weight loads depend on nothing an earlier kernel writes either: they are issued ahead of the wait on that kernel.
+  const int warp = warp_index();
   const int lane = threadIdx.x & 31;
-  // With static sizes (no device-side row count or K) the weight loads depend on nothing an earlier kernel writes:
-  // they are issued here, ahead of the wait on that kernel; the activation loads follow the wait.
-  const int tile_n = nt * BN;
+  const int n_base = nt * kFewBN;
+  const int tmem_cols = nb <= 32 ? 32 : nb <= 64 ? 64 : nb <= 128 ? 128 : 256;
   int early = 0;
   if (threadIdx.x == 0) {
-    for (int s = 0; s < C::STAGES; ++s) {
+    for (int s = 0; s < stages; ++s) {
       mbar_init(&full_bar[s], 1);
       mbar_init(&empty_bar[s], 1);
     }
@@ -93,25 +199,25 @@ gemm_skinny_kernel(const __grid_constant__ GemmArgs args, int* __restrict__ stat
     fence_mbar_init();
     tma_prefetch_desc(&p.tmA);
     tma_prefetch_desc(&p.tmB);
-    if (p.dyn == nullptr && p.M > mt * BM && p.K > 0 && (p.k0 & 7) == 0 && tile_n < p.N) {
+    if (p.dyn == nullptr && p.M > mt * nb && p.K > 0 && (p.k0 & 7) == 0 && n_base < p.N) {
       const int nkb_s = (p.K + BK - 1) / BK;
       const int b0 = static_cast<int>(static_cast<long>(nkb_s) * rank / splits);
       const int b1 = static_cast<int>(static_cast<long>(nkb_s) * (rank + 1) / splits);
-      early = min(b1 - b0, C::STAGES);
+      early = min(b1 - b0, stages);
       for (int j = 0; j < early; ++j) {
-        mbar_arrive_expect_tx(&full_bar[j], C::STAGE_BYTES);
-        tma_load_2d(smem + j * C::STAGE_BYTES + C::A_BYTES, &p.tmB, &full_bar[j], p.k0 + (b0 + j) * BK, tile_n);
+        mbar_arrive_expect_tx(&full_bar[j], stage_bytes);
+        tma_load_2d(smem + j * stage_bytes, &p.tmB, &full_bar[j], p.k0 + (b0 + j) * BK, n_base);
       }
     }
   }
   if (warp == 2) {
-    tmem_alloc(tmem_slot, BN);
+    tmem_alloc(tmem_slot, tmem_cols);
     tmem_relinquish();
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = warp_uniform(*tmem_slot);
   pdl_wait();
   pdl_launch_dependents();
 
@@ -123,98 +229,102 @@ gemm_skinny_kernel(const __grid_constant__ GemmArgs args, int* __restrict__ stat
     if (d2 >= 0) k0 = d2;
     if (d3 >= 0) K = d3;
   }
-  // a problem without rows on the device, or a column tile past N: nothing to do (uniform over the cluster)
-  M -= mt * BM;  // rows of this tile (the last row tile of a problem may be short, or empty on the device)
-  m0 += mt * BM;
-  if (M > BM) M = BM;
-  const bool live = M > 0 && K > 0 && nt * BN < p.N && WX_CHK(M <= A_ROWS && (k0 & 7) == 0, 2006, M, k0);
+  K = warp_uniform(K);
+  M = min(warp_uniform(M) - mt * nb, nb);  // rows of this tile (the last tile of a problem may be short, or empty on the device)
+  m0 += mt * nb;
+  // a tile without rows on the device, or a column tile past N: nothing to do (uniform over the cluster)
+  const bool live = M > 0 && K > 0 && n_base < p.N && WX_CHK((k0 & 7) == 0, 2006, M, k0);
 
   const int nkb = (K + BK - 1) / BK;
   const int kb0 = static_cast<int>(static_cast<long>(nkb) * rank / splits);
   const int kb1 = static_cast<int>(static_cast<long>(nkb) * (rank + 1) / splits);
   const int nblk = kb1 - kb0;  // this CTA's k blocks (0 when there are more CTAs than blocks: it contributes zeros)
-  const int n_base = nt * BN;
 
   if (!live) {
     // straight to the teardown: no cluster barrier is used by a cluster that does not work
   } else {
     if (warp == 0) {
-      if (lane == 0) {
-        for (int j = 0; j < nblk; ++j) {
-          const int s = j % C::STAGES;
-          const int use = j / C::STAGES;
-          if (use > 0 && !mbar_wait(&empty_bar[s], static_cast<uint32_t>(use - 1) & 1u, abort_flag)) break;
-          uint8_t* sA = smem + s * C::STAGE_BYTES;
+      // (one elected lane issues, the whole warp runs the loop: addresses and coordinates stay in uniform registers)
+      early = __shfl_sync(0xffffffffu, early, 0);
+      int s = 0;
+      uint32_t phase = 1;
+      for (int j = 0; j < nblk; ++j) {
+        if (j >= stages && !__all_sync(0xffffffffu, mbar_wait(&empty_bar[s], phase, abort_flag))) break;
+        if (elect_one()) {
+          uint8_t* sB = smem + s * stage_bytes;
           const int kc = k0 + (kb0 + j) * BK;
           if (j >= early) {  // (the first `early` weight slices are already on their way)
-            mbar_arrive_expect_tx(&full_bar[s], C::STAGE_BYTES);
-            tma_load_2d(sA + C::A_BYTES, &p.tmB, &full_bar[s], kc, n_base);  // the weight slice first: it comes from DRAM
+            mbar_arrive_expect_tx(&full_bar[s], stage_bytes);
+            tma_load_2d(sB, &p.tmB, &full_bar[s], kc, n_base);  // the weight slice first: it comes from DRAM
           }
-          tma_load_2d(sA, &p.tmA, &full_bar[s], kc, m0);
+          tma_load_2d(sB + kFewBBytes, &p.tmA, &full_bar[s], kc, m0);
+        }
+        if (++s == stages) {
+          s = 0;
+          phase ^= 1u;
         }
       }
     } else if (warp == 1) {
-      if (lane == 0) {
-        constexpr uint32_t idesc = make_idesc_bf16(BM, BN, false, false);
-        bool ok = true;
-        for (int j = 0; j < nblk; ++j) {
-          const int s = j % C::STAGES;
-          const int use = j / C::STAGES;
-          if (!mbar_wait(&full_bar[s], static_cast<uint32_t>(use) & 1u, abort_flag)) {
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          const uint32_t a_addr = smem_u32(smem + s * C::STAGE_BYTES);
-          const uint32_t b_addr = a_addr + C::A_BYTES;
+      // the whole warp runs the loop and one elected lane issues: the descriptors then live in uniform registers
+      const uint32_t idesc = make_idesc_bf16(kFewBN, nb, false, false);
+      const uint64_t dw0 = make_smem_desc_sw128(smem_u32(smem), 16, 1024);
+      const uint32_t stage16 = static_cast<uint32_t>(stage_bytes) >> 4;
+      bool ok = true;
+      int s = 0;
+      uint32_t phase = 0;
+      for (int j = 0; j < nblk; ++j) {
+        ok = __all_sync(0xffffffffu, mbar_wait(&full_bar[s], phase, abort_flag));
+        if (!ok) break;
+        tc_fence_after();
+        const uint64_t dw = dw0 + s * stage16, dx = dw + (kFewBBytes >> 4);
+        if (elect_one()) {
 #pragma unroll
-          for (int k = 0; k < BK / 16; ++k)
-            tc_mma_bf16(tmem_base, make_smem_desc_sw128(a_addr + k * 32, 16, 1024),
-                        make_smem_desc_sw128(b_addr + k * 32, 16, 1024), idesc, (j | k) != 0 ? 1u : 0u);
-          if (j + C::STAGES < nblk) tc_commit(&empty_bar[s]);  // only a stage that will be loaded again is handed back
+          for (int k = 0; k < BK / 16; ++k) tc_mma_bf16(tmem_base, dw + 2 * k, dx + 2 * k, idesc, (j | k) != 0 ? 1u : 0u);
+          if (j + stages < nblk) tc_commit(&empty_bar[s]);  // only a stage that will be loaded again is handed back
         }
-        if (ok && nblk > 0) tc_commit(tfull_bar);
+        if (++s == stages) {
+          s = 0;
+          phase ^= 1u;
+        }
       }
+      if (ok && nblk > 0 && elect_one()) tc_commit(tfull_bar);
+      __syncwarp();
     } else {
-      // ---- this CTA's partial tile: tensor memory -> shared memory (rows of this warp's lane quarter)
+      // ---- this CTA's partial tile: tensor memory (lane = output column, column = activation row) -> shared memory
       const int quarter = warp & 3;
-      if (quarter * 32 < A_ROWS && quarter * 32 < M) {
-        bool have = nblk > 0;
-        if (have) {
-          have = mbar_wait(tfull_bar, 0u, abort_flag);
-          tc_fence_after();
-        }
-        float* prow = partial + (quarter * 32 + lane) * C::PITCH;
-#pragma unroll
-        for (int c = 0; c < BN / 32; ++c) {
-          uint32_t r[32];
-          if (have) {
-            tmem_ld_32x32(tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + c * 32, r);
-            tmem_ld_wait();
-          } else {
-#pragma unroll
-            for (int i = 0; i < 32; ++i) r[i] = 0u;
-          }
-#pragma unroll
-          for (int q4 = 0; q4 < 8; ++q4)
-            *reinterpret_cast<uint4*>(prow + c * 32 + 4 * q4) = make_uint4(r[4 * q4], r[4 * q4 + 1], r[4 * q4 + 2], r[4 * q4 + 3]);
-        }
-        tc_fence_before();
+      const int half = (warp - 2) >> 2;  // two warps per lane quarter take alternate groups of 32 rows
+      bool have = nblk > 0;
+      if (have) {
+        have = mbar_wait(tfull_bar, 0u, abort_flag);
+        tc_fence_after();
       }
+      for (int r0 = half * 32; r0 < M; r0 += 64) {
+        uint32_t r[32];
+        if (have) {
+          tmem_ld_32x32(tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + r0, r);
+          tmem_ld_wait();
+        } else {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) r[i] = 0u;
+        }
+        float* dst = partial + r0 * kFewBN + quarter * 32 + lane;
+#pragma unroll
+        for (int i = 0; i < 32; ++i)
+          if (r0 + i < M) dst[i * kFewBN] = __uint_as_float(r[i]);
+      }
+      tc_fence_before();
     }
-    // What the epilogue of this thread's first piece will read from global memory (row map, residual, bias) is
-    // requested now, so that it arrives while the cluster barrier is being waited for.
-    const int pieces = M * (BN / 32);
+    // What the epilogue of this warp's first row will read from global memory is requested now, so that it arrives while
+    // the cluster barrier is being waited for.
+    const int n = n_base + lane * 4;
     {
-      const int i = static_cast<int>(threadIdx.x) * splits + rank;
-      if (i < pieces) {
-        const int r = i / (BN / 32);
-        const int n0 = n_base + (i - r * (BN / 32)) * 32;
+      const int r = rank + splits * warp;
+      if (r < M && n < p.N) {
         long drow = static_cast<long>(m0) + r;
         if (p.row_map != nullptr) drow = p.row_map[drow];
-        if (drow >= 0 && n0 < p.N) {
-          if (p.residual != nullptr) prefetch_l1(p.residual + drow * p.ldr + n0);
-          if (p.bias != nullptr) prefetch_l1(p.bias + n0);
+        if (drow >= 0) {
+          if (p.residual != nullptr) prefetch_l1(p.residual + drow * p.ldr + n);
+          if (p.bias != nullptr) prefetch_l1(p.bias + n);
         }
       }
     }
@@ -224,43 +334,27 @@ gemm_skinny_kernel(const __grid_constant__ GemmArgs args, int* __restrict__ stat
       cluster_arrive();
       cluster_wait();
     }
-    // ---- sum over the cluster and epilogue: piece i = (row i / 2, 32-column half i % 2) goes to CTA i % splits
-    const uint32_t partial_addr = smem_u32(partial);
-    for (int slot = threadIdx.x;; slot += kSkinnyThreads) {
-      const int i = slot * splits + rank;
-      if (i >= pieces) break;
-      const int r = i / (BN / 32);
-      const int c = i - r * (BN / 32);
-      const int n0 = n_base + c * 32;
-      if (n0 >= p.N) continue;
-      float v[32];
+    // ---- sum over the cluster and epilogue: row r goes to CTA r % splits, a row per warp at a time
+    const uint32_t partial_addr = smem_u32(partial) + lane * 16;
+    for (int r = rank + splits * warp; r < M; r += splits * kFewWarps) {
+      float4 v;
+      if (splits == 1) {
+        v = *reinterpret_cast<const float4*>(partial + r * kFewBN + lane * 4);
+      } else {
+        float4 x[kFewMaxSplits];
 #pragma unroll
-      for (int e = 0; e < 32; ++e) v[e] = 0.f;
-      const uint32_t off = static_cast<uint32_t>((r * C::PITCH + c * 32) * 4);
-      // two CTAs' pieces are requested before either is added (16 loads in flight); the sums keep the rank order
-      for (int s = 0; s < splits; s += 2) {
-        const bool two = s + 1 < splits;
-        const uint32_t base0 = mapa_u32(partial_addr + off, static_cast<uint32_t>(s));
-        const uint32_t base1 = mapa_u32(partial_addr + off, static_cast<uint32_t>(two ? s + 1 : s));
-        float4 x0[8], x1[8];
-#pragma unroll
-        for (int q4 = 0; q4 < 8; ++q4) x0[q4] = ld_cluster_f32x4(base0 + 16 * q4);
-#pragma unroll
-        for (int q4 = 0; q4 < 8; ++q4) x1[q4] = two ? ld_cluster_f32x4(base1 + 16 * q4) : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-        for (int q4 = 0; q4 < 8; ++q4) {
-          v[4 * q4] += x0[q4].x;
-          v[4 * q4 + 1] += x0[q4].y;
-          v[4 * q4 + 2] += x0[q4].z;
-          v[4 * q4 + 3] += x0[q4].w;
+        for (int s = 0; s < kFewMaxSplits; ++s) {
+          x[s] = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (s < splits) x[s] = ld_cluster_f32x4(mapa_u32(partial_addr + r * (kFewBN * 4), static_cast<uint32_t>(s)));
         }
-        if (two) {
+        v = x[0];
 #pragma unroll
-          for (int q4 = 0; q4 < 8; ++q4) {
-            v[4 * q4] += x1[q4].x;
-            v[4 * q4 + 1] += x1[q4].y;
-            v[4 * q4 + 2] += x1[q4].z;
-            v[4 * q4 + 3] += x1[q4].w;
+        for (int s = 1; s < kFewMaxSplits; ++s) {
+          if (s < splits) {
+            v.x += x[s].x;
+            v.y += x[s].y;
+            v.z += x[s].z;
+            v.w += x[s].w;
           }
         }
       }
@@ -271,10 +365,10 @@ gemm_skinny_kernel(const __grid_constant__ GemmArgs args, int* __restrict__ stat
         drow = mapped;
       }
       if (!WX_CHK(drow >= 0 && (p.d_rows == 0 || drow < p.d_rows), 2007, drow, p.d_rows)) continue;
-      epilogue_chunk(p, v, drow, n0, false);
+      epilogue_quad(p, v, drow, n);
     }
-    __syncthreads();
     if (splits > 1) {  // nobody leaves while a peer may still read its tile
+      __syncthreads();
       cluster_arrive();
       cluster_wait();
     }
@@ -285,39 +379,87 @@ gemm_skinny_kernel(const __grid_constant__ GemmArgs args, int* __restrict__ stat
   if (threadIdx.x == 0 && *abort_flag) atomicExch(status, 1);
   if (warp == 2) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, BN);
+    tmem_dealloc(tmem_base, tmem_cols);
   }
 }
 
-template <int A_ROWS, int BN>
-int launch_skinny_t(const GemmArgs& args, int tiles, int splits, cudaStream_t stream, int* status) {
-  using C = SkinnyCfg<A_ROWS, BN>;
-  auto kern = gemm_skinny_kernel<A_ROWS, BN>;
+constexpr int kFewSmemMax = 227 * 1024;
+constexpr int kFewSmemHalf = 113 * 1024;  // two CTAs of this size share an SM
+constexpr int kFewSmemExtra = 1024 + 512;
+
+inline int few_smem(const FewShape& sh) { return sh.stages * (kFewBBytes + sh.nb * BK * 2) + kFewSmemExtra; }
+
+// Clusters of this shape that the device holds at once (-1: none). Stages fill half or all of an SM's shared memory, so
+// there are two answers per cluster size.
+inline int few_capacity(const FewShape& sh) {
+  static std::atomic<int> cap[2][kFewMaxSplits + 1];
+  std::atomic<int>& slot = cap[few_smem(sh) <= kFewSmemHalf ? 0 : 1][sh.splits];
+  int n = slot.load(std::memory_order_relaxed);
+  if (n != 0) return n;
+  if (cudaFuncSetAttribute(gemm_few_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFewSmemMax) != cudaSuccess) {
+    cudaGetLastError();
+    return -1;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(sh.splits * num_sms()));
+  cfg.blockDim = dim3(kFewThreads);
+  cfg.dynamicSmemBytes = few_smem(sh) <= kFewSmemHalf ? kFewSmemHalf : kFewSmemMax;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = static_cast<unsigned>(sh.splits);
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  if (cudaOccupancyMaxActiveClusters(&n, gemm_few_kernel, &cfg) != cudaSuccess) {
+    cudaGetLastError();
+    n = 0;
+  }
+  if (n < 1) n = -1;
+  slot.store(n, std::memory_order_relaxed);
+  return n;
+}
+
+// Shape of a launch whose largest problem has `max_m` rows, `col_tiles` column tiles in all and at least `min_nkb` k steps.
+// Up to 64 rows the stages take half of an SM's shared memory: two CTAs then stream weights side by side, and under
+// programmatic dependent launch the CTAs of the next such GEMM sit beside this one's and request their weights while this
+// one finishes. K is split over as many CTAs as keep every cluster resident with five k steps or more each; up to 64 rows
+// in powers of two (2048 x 2048, 32 rows: 8.0 us with 4, 7.9 with 8; as dependent launches 5.9 and 6.0, 6.6 with 5 or 6).
+inline FewShape few_shape(int max_m, long col_tiles, int min_nkb) {
+  FewShape sh;
+  const int mtiles = (max_m + kFewMaxRows - 1) / kFewMaxRows;
+  sh.nb = ((max_m + mtiles - 1) / mtiles + 15) & ~15;
+  const int stage = kFewBBytes + sh.nb * BK * 2;
+  const int budget = (sh.nb <= 64 ? kFewSmemHalf : kFewSmemMax) - kFewSmemExtra;
+  sh.stages = budget / stage;
+  if (sh.stages > 8) sh.stages = 8;
+  const long tiles = col_tiles * ((max_m + sh.nb - 1) / sh.nb);
+  sh.splits = 1;
+  for (int s = 2; s <= kFewMaxSplits; s += sh.nb <= 64 ? s : 1) {
+    FewShape t = sh;
+    t.splits = s;
+    if (min_nkb < 5 * s || few_capacity(t) < tiles) break;
+    sh.splits = s;
+  }
+  return sh;
+}
+
+int launch_few(const GemmCall* calls, int ncalls, const FewShape& sh, cudaStream_t stream, int* status) {
+  // the partial tile reuses the ring
+  if (sh.stages < 2 || sh.nb * kFewBN * 4 > few_smem(sh) - kFewSmemExtra || few_smem(sh) > kFewSmemMax) return -12;
+  GemmArgs args;
+  const int rc = fill_args(args, calls, ncalls, kFewBN, sh.nb);
+  if (rc != 0) return rc;
+  long tiles = 0;
+  for (int i = 0; i < ncalls; ++i)
+    tiles += static_cast<long>((calls[i].N + kFewBN - 1) / kFewBN) * ((calls[i].M + sh.nb - 1) / sh.nb);
   static bool attr_set = false;
   if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
+    cudaError_t e = cudaFuncSetAttribute(gemm_few_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFewSmemMax);
     if (e != cudaSuccess) return static_cast<int>(e);
     attr_set = true;
   }
-  return static_cast<int>(launch_kernel_cluster(kern, dim3(static_cast<unsigned>(tiles * splits)), dim3(kSkinnyThreads),
-                                                C::SMEM_BYTES, stream, static_cast<unsigned>(splits), args, status, splits));
-}
-
-// Rows staged per k step for a launch whose largest problem has `max_m` rows.
-inline int skinny_rows(int max_m) { return max_m <= 32 ? 32 : max_m <= 64 ? 64 : 128; }
-
-// CTAs per cluster: as many as keep all clusters in one wave (a power of two, at most 8), each with two k blocks or more.
-inline int skinny_splits(long tiles, int min_nkb, int sms) {
-  int s = 1;
-  while (s * 2 <= kSkinnyMaxSplits && tiles * (s * 2) <= sms && min_nkb >= 2 * (s * 2)) s *= 2;
-  return s;
-}
-
-int launch_skinny(const GemmArgs& args, int a_rows, int bn, int tiles, int splits, cudaStream_t stream, int* status) {
-  if (bn == kMidBN) return launch_skinny_t<128, kMidBN>(args, tiles, splits, stream, status);
-  if (a_rows == 32) return launch_skinny_t<32, kSkinnyBN>(args, tiles, splits, stream, status);
-  if (a_rows == 64) return launch_skinny_t<64, kSkinnyBN>(args, tiles, splits, stream, status);
-  return launch_skinny_t<128, kSkinnyBN>(args, tiles, splits, stream, status);
+  return static_cast<int>(launch_kernel_cluster(gemm_few_kernel, dim3(static_cast<unsigned>(tiles * sh.splits)), dim3(kFewThreads),
+                                                few_smem(sh), stream, static_cast<unsigned>(sh.splits), args, status, sh));
 }
 
 }  // namespace
