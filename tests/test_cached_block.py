@@ -1,0 +1,77 @@
+"""One host call per layer of a cached step (``block_cached`` in csrc/blocks.cpp) and the per-step decoding tables."""
+import pytest
+import torch
+
+from wallx_b200.ops import functional as F_
+
+
+@pytest.mark.parametrize("lens,steps", [([1], 1), ([3, 17, 9], 5)])
+def test_decode_tables_equal_the_ones_built_step_by_step(lens, steps):
+    caps = [n + steps + 2 for n in lens]
+    starts = [sum(caps[:i]) for i in range(len(caps))]
+    ds = F_.DecodeSteps(starts, lens, steps, sum(caps), "cpu")
+    for i in range(steps):
+        now = [n + i + 1 for n in lens]
+        want = F_.AttnMeta(list(range(len(lens) + 1)), "cpu", causal=True, k_starts=starts, k_lens=now, k_rows=sum(caps))
+        got = ds.meta(i, 16)
+        assert torch.equal(got.device_tables("cpu")[0], want.device_tables("cpu")[0])
+        assert got.device_tables("cpu")[1].shape == want.device_tables("cpu")[1].shape
+        assert torch.equal(got.row_tiles("cpu", 16), want.row_tiles("cpu", 16))
+        assert got.cache_rows.tolist() == [s + n - 1 for s, n in zip(starts, now)]
+        assert (got.k_ranges, got.max_k, got.cu_k_host) == (want.k_ranges, want.max_k, want.cu_k_host)
+
+
+def _model(mlp_moe=True):
+    from wallx_b200.config import tiny_config
+    from wallx_b200.data.synthetic import make_processor
+    from wallx_b200.models import Qwen2_5_VLMoEForAction
+
+    cfg = tiny_config()
+    proc = make_processor(cfg, 16)
+    torch.manual_seed(0)
+    model = Qwen2_5_VLMoEForAction(cfg, processor=proc).to(torch.bfloat16).cuda()
+    model.init_weights(seed=1)
+    return cfg, proc, model.eval()
+
+
+def _run_layers(model, cfg, x, meta_args, plan, single, fused, monkeypatch):
+    from wallx_b200.models.llm import KVCache, StepContext
+    from wallx_b200.ops import blocks as BK
+    from wallx_b200.ops.gemm import inference_kernels
+
+    monkeypatch.setattr(BK, "ENABLED", fused)
+    cu, lens, mode = meta_args
+    cache = KVCache(cfg.num_hidden_layers, [n + 4 for n in lens], cfg.num_key_value_heads * cfg.head_dim, x.device, x.dtype)
+    g = torch.Generator("cuda").manual_seed(3)
+    for b in cache.buffers:
+        b.normal_(generator=g)
+    rows = torch.cat([cache.slot_rows(i, n - (cu[i + 1] - cu[i]), cu[i + 1] - cu[i]) for i, n in enumerate(lens)])
+    meta = F_.AttnMeta(cu, x.device, causal=True, cache_rows=rows, k_starts=cache.offsets[:-1], k_lens=lens, k_rows=cache.offsets[-1])
+    pos = torch.arange(x.shape[0], device=x.device).reshape(1, -1).expand(3, -1)
+    cos, sin = model.model.rotary(pos)
+    if plan is not None:
+        plan.single_expert = single
+    with torch.no_grad(), inference_kernels():
+        y = model.model(x, StepContext(meta, cos, sin, plan, cache=cache, cache_mode=mode))
+    return y, cache.buffers
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("cu,lens,mode", [([0, 1], [9], "step"), ([0, 1, 2, 3], [4, 200, 130], "step"), ([0, 16, 32], [40, 60], "step"),
+                                          ([0, 300, 317], [300, 17], "prefill")])
+@pytest.mark.parametrize("experts", ["first", "second", "mixed"])
+def test_one_call_per_layer_gives_the_bits_of_the_operator_path(cu, lens, mode, experts, monkeypatch):
+    cfg, _, model = _model()
+    T = cu[-1]
+    x = torch.randn(T, cfg.hidden_size, device="cuda", generator=torch.Generator("cuda").manual_seed(5)).to(torch.bfloat16)
+    types = {"first": torch.zeros(T), "second": torch.ones(T), "mixed": torch.arange(T) % 2}[experts].to(torch.int32).cuda()
+    plan = F_.make_route_plan(types, cfg.num_experts)
+    single = {"first": 0, "second": 1, "mixed": None}[experts]
+    a, ca = _run_layers(model, cfg, x, (cu, lens, mode), plan, single, True, monkeypatch)
+    b, cb = _run_layers(model, cfg, x, (cu, lens, mode), plan, single, False, monkeypatch)
+    torch.cuda.synchronize()
+    from wallx_b200.ops import gemm as G
+
+    G.check_status()
+    assert torch.equal(a, b)
+    assert all(torch.equal(u, v) for u, v in zip(ca, cb))

@@ -23,6 +23,7 @@
 
 #include "attention.h"
 #include "bind_common.h"
+#include "decode.h"
 #include "gemm.h"
 #include "kernels.h"
 
@@ -70,10 +71,10 @@ wxb::GemmTuple to_tuple(const Spec& s) {
                         0, 0);
 }
 
-void launch_plain(const Spec* specs, int n, int* status) {
+void launch_plain(const Spec* specs, int n, int* status, int force_bn = 0) {
   wx::GemmCall cs[2];
   for (int i = 0; i < n; ++i) wxb::fill_call(cs[i], to_tuple(specs[i]));
-  WX_RC(wx::gemm_launch(cs, n, cur(), status, 0), "gemm_launch");
+  WX_RC(wx::gemm_launch(cs, n, cur(), status, force_bn), "gemm_launch");
 }
 
 void launch_gathered(const Spec* specs, const WTuple* const* ws, int n, int* status) {
@@ -354,6 +355,119 @@ std::vector<Tensor> block_fwd(const Tensor& x, const Tensor& ln1_w, const WTuple
   return {out, y1, rstd1, qkv, o_attn, lse, x2, rstd2, xn, gu, h};
 }
 
+bool operand_ok(const Tensor& t) {
+  return t.is_cuda() && t.scalar_type() == at::kBFloat16 && t.dim() == 2 && t.stride(1) == 1 && (t.stride(0) & 7) == 0 &&
+         (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0;
+}
+
+// One layer of a cached step (prefix pass into the key-value cache, denoise step, token decoding), inference only:
+// rotary writes the rows' cache slots and attention runs over the cache. `attn` chooses the kernel as
+// ops.functional.attention_decode does (2: attn_cached with `tiles`, 1: attn_decode, 0: attn_fwd). `ffn` holds one
+// (gate_up, down) pair when all rows go to one FFN, else all experts' with the routing plan. Returns None when an operand
+// would need a copy first: the caller then takes the operator path.
+c10::optional<Tensor> block_cached(const Tensor& x, const Tensor& ln1_w, const Tensor& w_qkv, const OptT& b_qkv, const Tensor& cos_t,
+                                   const Tensor& sin_t, const Tensor& cache_rows, Tensor& cache, const Tensor& qtab,
+                                   const Tensor& ktab, const OptT& tiles, int64_t attn, int64_t max_keys, int64_t hq, int64_t hkv,
+                                   int64_t d, double scale, bool has_bidir, const Tensor& w_o, const OptT& b_o, const Tensor& ln2_w,
+                                   double eps, const std::vector<Tensor>& ffn, const OptT& dest, const OptT& seg, const OptT& inv,
+                                   int64_t rows, bool infer) {
+  const int64_t T = x.size(0), H = x.size(1), W = (hq + 2 * hkv) * d;
+  if (T == 0 || !operand_ok(x) || !x.is_contiguous() || !operand_ok(w_qkv) || !operand_ok(w_o) || !operand_ok(cache) ||
+      w_qkv.size(0) != W || w_qkv.size(1) != H || w_o.size(0) != H || w_o.size(1) != hq * d || cache.size(1) != 2 * hkv * d)
+    return c10::nullopt;
+  for (const Tensor& w : ffn)
+    if (!operand_ok(w)) return c10::nullopt;
+  for (const Tensor* w : {&ln1_w, &ln2_w})
+    if (!w->is_cuda() || w->scalar_type() != at::kBFloat16 || !w->is_contiguous() || w->numel() != H) return c10::nullopt;
+  if (!cos_t.is_cuda() || cos_t.scalar_type() != at::kFloat || sin_t.scalar_type() != at::kFloat || !cos_t.is_contiguous() ||
+      !sin_t.is_contiguous() || cos_t.size(0) != T || sin_t.size(0) != T || cos_t.size(1) != d || !cache_rows.is_cuda() ||
+      cache_rows.scalar_type() != at::kLong || !cache_rows.is_contiguous() || cache_rows.numel() != T)
+    return c10::nullopt;
+  TORCH_CHECK(qtab.scalar_type() == at::kInt && qtab.is_contiguous() && qtab.size(0) == T && qtab.size(1) == 4 &&
+                  ktab.scalar_type() == at::kInt && ktab.is_contiguous() && ktab.size(0) == cache.size(0) && ktab.size(1) == 4,
+              "block_cached: attention tables must be int32 [rows, 4]");
+  const bool moe = dest.has_value() && dest->defined();
+  const int n_exp = static_cast<int>(ffn.size() / 2);
+  TORCH_CHECK(ffn.size() >= 2 && ffn.size() % 2 == 0 && (moe || n_exp == 1), "block_cached: ffn weights come in (gate_up, down) pairs");
+  c10::cuda::CUDAGuard guard(x.device());
+  int* status = wxb::status_tensor(x.device()).data_ptr<int>();
+  const int force = infer ? 18 : 0;
+
+  Tensor qkv = empty_bf16(T, W, x);
+  {
+    Spec s;
+    s.a = norm_fwd(x, ln1_w, eps, OptT(), 0, false).first;
+    s.b = w_qkv;
+    s.out = qkv;
+    s.bias = b_qkv;
+    launch_plain(&s, 1, status, force);
+  }
+  WX_RC(wx::rope_cache(qkv.data_ptr(), cos_t.data_ptr<float>(), sin_t.data_ptr<float>(), cache_rows.data_ptr<int64_t>(),
+                       cache.data_ptr(), T, W, hq, hkv, d, cache.stride(0), cache.size(0), cur()),
+        "rope_cache");
+  Tensor o = empty_bf16(T, hq * d, x);
+  {
+    Tensor k = cache.narrow(1, 0, hkv * d), v = cache.narrow(1, hkv * d, hkv * d);
+    wx::AttnShape s = attn_shape(qkv, hq, hkv, d, scale, has_bidir, false);
+    s.Tk = cache.size(0);
+    s.ld_k = s.ld_v = cache.stride(0);
+    if (attn == 2) {
+      TORCH_CHECK(tiles.has_value() && tiles->is_cuda() && tiles->scalar_type() == at::kInt && tiles->is_contiguous() &&
+                      tiles->dim() == 2 && tiles->size(1) == 4, "block_cached: tile table");
+      WX_RC(wx::attn_cached(s, qkv.data_ptr(), k.data_ptr(), v.data_ptr(), qtab.data_ptr(), ktab.data_ptr(), tiles->data_ptr(),
+                            tiles->size(0), max_keys, o.data_ptr(), o.stride(0), cur(), status),
+            "attn_cached");
+    } else if (attn == 1) {
+      WX_RC(wx::attn_decode(qkv.data_ptr(), qkv.stride(0), k.data_ptr(), k.stride(0), v.data_ptr(), v.stride(0), qtab.data_ptr(),
+                            ktab.data_ptr(), o.data_ptr(), o.stride(0), T, cache.size(0), hq, hkv, d, static_cast<float>(scale),
+                            max_keys, cur()),
+            "attn_decode");
+    } else {
+      Tensor lse = at::empty({hq, T}, x.options().dtype(at::kFloat));
+      WX_RC(wx::attn_fwd(s, qkv.data_ptr(), k.data_ptr(), v.data_ptr(), qtab.data_ptr(), ktab.data_ptr(), o.data_ptr(), o.stride(0),
+                         lse.data_ptr<float>(), cur(), status),
+            "attn_fwd");
+    }
+  }
+  Tensor x2 = empty_bf16(T, H, x), out = empty_bf16(T, H, x);
+  {
+    Spec s;
+    s.a = o;
+    s.b = w_o;
+    s.out = x2;
+    s.bias = b_o;
+    s.residual = x;
+    launch_plain(&s, 1, status, force);
+  }
+  Tensor xn = norm_fwd(x2, ln2_w, eps, dest, rows, false).first;
+  const int64_t hrows = moe ? rows : T;
+  int64_t wmax = 0;
+  for (int e = 0; e < n_exp; ++e) wmax = std::max<int64_t>(wmax, ffn[2 * e].size(0));
+  Tensor h = empty_bf16(hrows, wmax / 2, x);
+  for (int half = 0; half < 2; ++half) {  // gate/up, then down; two experts per launch
+    for (int e0 = 0; e0 < n_exp; e0 += 2) {
+      Spec sp[2];
+      const int n = std::min(2, n_exp - e0);
+      for (int i = 0; i < n; ++i) {
+        const Tensor& w = ffn[2 * (e0 + i) + half];
+        Spec& s = sp[i];
+        s.b = w;
+        s.a = half ? h.narrow(1, 0, w.size(1)) : xn;
+        s.out = half ? out : h;
+        if (moe) {
+          s.M = rows;
+          s.dyn = seg->select(0, e0 + i);
+          if (half) s.row_map = inv;
+        }
+        if (half) s.residual = x2;
+        else s.flags = wx::GEMM_ACT_SWIGLU | (moe ? wx::GEMM_ZERO_PAD_ROWS : 0);
+      }
+      launch_plain(sp, n, status, force);
+    }
+  }
+  return out;
+}
+
 // Backward. Weight gradients go into the sinks (accumulate) where a weight has one; otherwise they are returned.
 // Returns {dx, d ln1_w, d ln2_w, d b_qkv, d b_o, d b_gu, d b_dn, dW qkv, dW o, dW ffn[0], dW ffn[1], ...}
 // with undefined tensors where nothing is due (no bias, or the gradient went into a sink).
@@ -569,6 +683,7 @@ std::vector<Tensor> block_bwd(const Tensor& dout_in, const Tensor& x, const Tens
 
 void register_block_bindings(pybind11::module_& m) {
   m.def("block_fwd", &block_fwd, "one pre-norm attention + FFN block, forward: every kernel enqueued by one host call");
+  m.def("block_cached", &block_cached, "one layer of a cached step (inference), or None when an operand needs a copy first");
   m.def("block_bwd", &block_bwd, "backward of block_fwd");
   m.def("block_launch_count", []() { return g_launches.load(); }, "kernels launched by block_fwd / block_bwd so far");
 }

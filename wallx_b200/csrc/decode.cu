@@ -19,17 +19,15 @@
 #include "launch.h"
 #include "ptx.cuh"
 
-#include <atomic>
-
 #include <cuda_bf16.h>
 
 namespace wx {
 
 namespace {
-std::atomic<bool> g_pdl{false};
+thread_local bool g_pdl = false;
 }  // namespace
-bool pdl_enabled() { return g_pdl.load(std::memory_order_relaxed); }
-void pdl_set(bool on) { g_pdl.store(on, std::memory_order_relaxed); }
+bool pdl_enabled() { return g_pdl; }
+void pdl_set(bool on) { g_pdl = on; }
 
 namespace {
 

@@ -4,10 +4,9 @@
 // Such a product reads far more weight than anything else, and what limits it is the time one SM needs for its share:
 //   * the roles of the operands are swapped. The 128 rows of the MMA are output columns (a slice of the weight) and the
 //     activation rows are its N, so a 64-wide k step stages 16 KB of weight and `nb` x 128 bytes of activations and the
-//     tensor core reads exactly that. (With the activations as the 128-row operand, 32 rows cost as much as 128 and a
-//     weight slice of 64 rows cost 0.1 us per k step whatever arrived.)
+//     tensor core reads exactly that. (With the activations as the 128-row operand, 32 rows cost as much as 128.)
 //   * one *cluster* of `splits` CTAs per 128 output columns, CTA r of the cluster owning the k blocks
-//     [nkb * r / splits, nkb * (r + 1) / splits): 2048 x 2048 runs as 16 clusters of 8, four k blocks per CTA.
+//     [nkb * r / splits, nkb * (r + 1) / splits): 2048 x 2048 runs as 16 clusters of 4, eight k blocks per CTA.
 //   * every CTA leaves its fp32 partial tile in its own shared memory as rows of 128 output columns; after a cluster
 //     barrier the rows are dealt to the warps of the cluster, which add the partials in rank order through distributed
 //     shared memory (a fixed order: results do not depend on timing), a whole 512-byte row per load, and run the epilogue

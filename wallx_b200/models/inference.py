@@ -15,7 +15,9 @@ evaluations. The Euler loop can be captured in a CUDA graph (``use_cuda_graph=Tr
 """
 from __future__ import annotations
 
+import contextlib
 import os
+import threading
 from typing import Dict, List, Optional
 
 import torch
@@ -34,6 +36,30 @@ def _ids_of(model, name, default):
         return default if v is None else v
     except Exception:
         return default
+
+
+_pdl_region = threading.local()
+
+
+class _dependent_launches(contextlib.ContextDecorator):
+    """Programmatic dependent launch of the inference kernels issued by this thread (csrc/launch.h): each one's prologue
+    overlaps the tail of the kernel before it. ``WALLX_PDL=0`` leaves it off."""
+
+    def __enter__(self):
+        from ..ops import _ext
+
+        C = _ext.get(required=False) if os.environ.get("WALLX_PDL", "1") == "1" else None
+        state = _pdl_region.__dict__.setdefault("stack", [])
+        state.append((C, C.pdl_enabled() if C is not None else False))
+        if C is not None:
+            C.set_pdl(True)
+        return self
+
+    def __exit__(self, *exc):
+        C, before = _pdl_region.stack.pop()
+        if C is not None:
+            C.set_pdl(before)
+        return False
 
 
 class FlowSampler:
@@ -205,6 +231,7 @@ class FlowSampler:
         return static_out.clone()
 
 
+@_dependent_launches()
 @inference_kernels()
 @torch.no_grad()
 def predict_flow(model, pred_horizon=None, action_dim=None, input_ids=None, action_chunk=None, dataset_names=None,
@@ -223,18 +250,6 @@ def predict_flow(model, pred_horizon=None, action_dim=None, input_ids=None, acti
         out["gt_action"] = model.action_preprocessor.normalizer_action.unnormalize_data(
             action_chunk.to(sampler.device).float(), names)
     return out
-
-
-def _pdl_switch(on: bool):
-    """Turn programmatic dependent launch of the small inference kernels on (when the extension is there) and return
-    the setter, so that the caller can turn it off again."""
-    from ..ops import _ext
-
-    C = _ext.get(required=False)
-    if C is None or not hasattr(C, "set_pdl"):
-        return lambda _on: None
-    C.set_pdl(bool(on))
-    return C.set_pdl
 
 
 class FlowEngine:
@@ -292,10 +307,7 @@ class FlowEngine:
         with torch.no_grad():
             self._run()  # eager warm-up: builds every cached table before capture
             if use_cuda_graph and dev.type == "cuda":
-                # Inside the graph the small kernels of the denoise loop are launched as programmatic dependents:
-                # each one's prologue overlaps the tail of the kernel before it (csrc/launch.h).
-                pdl = _pdl_switch(os.environ.get("WALLX_PDL", "1") == "1")
-                try:
+                with _dependent_launches():
                     torch.cuda.synchronize(dev)
                     side = torch.cuda.Stream(device=dev)
                     side.wait_stream(torch.cuda.current_stream(dev))
@@ -306,8 +318,6 @@ class FlowEngine:
                     with torch.cuda.graph(g):
                         self._run()
                     self.graph = g
-                finally:
-                    pdl(False)
 
     def _layout_signature(self, ids_host: torch.Tensor) -> torch.Tensor:
         sig = torch.zeros_like(ids_host, dtype=torch.int8)
@@ -393,29 +403,31 @@ class _Decoder:
         h = model.model(emb, ctx)
         last = torch.tensor([c - 1 for c in pack.cu[1:]], device=dev)
         self.last_hidden = h.index_select(0, last)
+        # ---- tables and rotary values of every later step
+        n = max(max_new_tokens - 1, 1)
+        self.steps = F_.DecodeSteps(self.cache.offsets[:B], self.lens, n, self.cache.offsets[-1], dev)
+        pos = (self.next_pos.reshape(1, B) + torch.arange(n, device=dev).reshape(n, 1)).reshape(1, -1).expand(3, n * B)
+        cos, sin = model.model.rotary(pos)
+        self.cos, self.sin = cos.reshape(n, B, -1), sin.reshape(n, B, -1)
+        self.plan = None
+        if cfg.mlp_moe:  # every row goes through the VLM expert: no grouping, so no routing tables
+            self.plan = F_.RoutePlan(None, None, None, None, 0)
+            self.plan.single_expert = 0
+        self.done = 0
 
     def logits(self) -> torch.Tensor:
         return F_.linear(self.last_hidden, self.model.lm_head.weight).float()
 
     def step(self, tokens: torch.Tensor) -> None:
         """Append one token per sample and compute the hidden state at it."""
-        m, cfg, B, dev = self.model, self.model.config, self.B, self.dev
-        emb = m.model.embed_tokens(tokens)
-        rows = torch.cat([self.cache.slot_rows(b, self.lens[b], 1) for b in range(B)])
-        self.lens = [l + 1 for l in self.lens]
-        meta = F_.AttnMeta(list(range(B + 1)), dev, causal=True, cache_rows=rows,
-                           k_starts=[self.cache.offsets[b] for b in range(B)], k_lens=self.lens,
-                           k_rows=self.cache.offsets[-1])
-        pos3 = self.next_pos.view(1, B).expand(3, B)
-        self.next_pos = self.next_pos + 1
-        cos, sin = m.model.rotary(pos3)
-        plan = F_.make_route_plan(torch.zeros(B, dtype=torch.int32, device=dev), cfg.num_experts) if cfg.mlp_moe else None
-        if plan is not None:
-            plan.single_expert = 0
-        ctx = StepContext(meta, cos, sin, plan, cache=self.cache, cache_mode="step")
-        self.last_hidden = m.model(emb, ctx)
+        cfg, i = self.model.config, self.done
+        meta = self.steps.meta(i, max(1, 128 * cfg.num_key_value_heads // cfg.num_attention_heads))
+        ctx = StepContext(meta, self.cos[i], self.sin[i], self.plan, cache=self.cache, cache_mode="step")
+        self.last_hidden = self.model.model(self.model.model.embed_tokens(tokens), ctx)
+        self.done = i + 1
 
 
+@_dependent_launches()
 @inference_kernels()
 @torch.no_grad()
 def generate(model, input_ids, max_new_tokens: int = 100, do_sample: bool = False, temperature: float = 1.0,

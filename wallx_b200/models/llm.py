@@ -150,6 +150,21 @@ class DecoderLayer(nn.Module):
                 self.post_attention_layernorm.weight, ffn_w, None, None, meta=ctx.meta, cos=ctx.cos, sin=ctx.sin,
                 n_rot=a.num_heads + a.num_kv_heads, hq=a.num_heads, hkv=a.num_kv_heads, d=a.head_dim,
                 eps=self.input_layernorm.variance_epsilon, plan=plan)
+        if ctx.cache is not None and ctx.cache_mode != "none" and BK.usable(x) and self._plain_modules():
+            a = self.self_attn
+            single = None if self.moe is None else ctx.plan.single_expert
+            if self.moe is None:
+                ffn_w, plan = self.mlp.weights(), None
+            elif single is not None:  # every token of this call belongs to one expert: a plain FFN, no grouping of rows
+                ffn_w, plan = self.moe.experts[single].weights(), None
+            else:
+                ffn_w, plan = [w for e in self.moe.experts for w in e.weights()], ctx.plan
+            y = BK.cached_block(x, self.input_layernorm.weight, a.qkv_proj.weight, a.qkv_proj.bias, a.o_proj.weight, a.o_proj.bias,
+                                self.post_attention_layernorm.weight, ffn_w, meta=ctx.meta, cos=ctx.cos, sin=ctx.sin,
+                                cache=ctx.cache.buffers[a.layer_idx], hq=a.num_heads, hkv=a.num_kv_heads, d=a.head_dim,
+                                eps=self.input_layernorm.variance_epsilon, plan=plan)
+            if y is not None:
+                return y
         x = self.self_attn(self.input_layernorm(x), ctx, residual=x)
         if self.moe is not None and ctx.plan.single_expert is not None and not torch.is_grad_enabled():
             # every token of this call belongs to one expert (known on the host): a plain FFN, no grouping of rows

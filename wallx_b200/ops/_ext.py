@@ -150,7 +150,7 @@ class LaunchCounter:
                 n = 3 if a[11] == a[12] else 5
             if name in ("read_status", "status_tensor", "block_launch_count"):
                 n = 0
-            if name in ("block_fwd", "block_bwd"):  # one host call, many kernels: the C++ side counts them
+            if name in ("block_fwd", "block_bwd", "block_cached"):  # one host call, many kernels: the C++ side counts them
                 before = self._mod.block_launch_count()
                 out = fn(*a, **k)
                 n = self._mod.block_launch_count() - before

@@ -141,3 +141,27 @@ def transformer_block(x: torch.Tensor, ln1_w, w_qkv, b_qkv, w_o, b_o, ln2_w, ffn
     scale = scale if scale is not None else 1.0 / math.sqrt(d)
     cfg = (meta, cos, sin, n_rot, hq, hkv, d, scale, eps, plan)
     return _BlockFn.apply(x.contiguous(), ln1_w, w_qkv, b_qkv, w_o, b_o, ln2_w, b_gu, b_dn, cfg, *ffn_w)
+
+
+def cached_block(x: torch.Tensor, ln1_w, w_qkv, b_qkv, w_o, b_o, ln2_w, ffn_w: Sequence[torch.Tensor], *, meta: F_.AttnMeta,
+                 cos, sin, cache: torch.Tensor, hq: int, hkv: int, d: int, eps: float,
+                 plan: Optional[F_.RoutePlan] = None) -> Optional[torch.Tensor]:
+    """One layer of a cached step as one host call: the kernels of the operator path (rotary with the cache write, attention
+    over the cache), same arguments, same bits. Every layer of a denoise or decoding step costs the host seven autograd
+    functions otherwise, twice what the device needs. None: the operator path has to serve the call (autograd on, row-sharded
+    weights, operands that need a copy)."""
+    weights = (w_qkv, w_o, *ffn_w)
+    if not F_.cached_step_kernels_usable(x, d) or any(F_._shard_of(w) is not None for w in weights):
+        return None
+    import math
+
+    from .gemm import _inference_launch
+
+    C = _ext.get()
+    kind = F_.cached_attention_kind(meta, x.shape[0], hq, hkv, d)
+    qtab, ktab = meta.device_tables(x.device)
+    return C.block_cached(x, ln1_w, w_qkv, b_qkv, cos, sin, meta.cache_rows, cache, qtab, ktab,
+                          meta.row_tiles(x.device, 128 // (hq // hkv)) if kind == 2 else None, kind, int(meta.max_k), hq, hkv, d,
+                          1.0 / math.sqrt(d), F_._attn_flags(meta)[0], w_o, b_o, ln2_w, eps, list(ffn_w),
+                          plan.dest if plan is not None else None, plan.seg if plan is not None else None,
+                          plan.inv if plan is not None else None, int(plan.rows) if plan is not None else 0, _inference_launch())

@@ -11,6 +11,7 @@ routing uses 128-row aligned segments so that forward, dgrad and wgrad are all t
 """
 from __future__ import annotations
 
+import copy
 import math
 import os
 from typing import Optional, Sequence, Tuple
@@ -677,6 +678,33 @@ class AttnMeta:
         return t
 
 
+class DecodeSteps:
+    """Tables of every step of token-by-token decoding (one new row per sequence, step ``i`` seeing ``lens[b] + i + 1`` keys
+    of the cache slot at ``starts[b]``), built and uploaded once instead of step by step."""
+
+    def __init__(self, starts: Sequence[int], lens: Sequence[int], steps: int, k_rows: int, device):
+        B = len(starts)
+        self.starts, self.lens, self.k_rows = list(starts), list(lens), k_rows
+        self.base = AttnMeta(list(range(B + 1)), device, causal=True, k_starts=starts, k_lens=[l + 1 for l in lens], k_rows=k_rows)
+        lo = torch.tensor(self.starts, dtype=torch.int32).reshape(1, B).expand(steps, B)
+        hi = lo + torch.tensor(self.lens, dtype=torch.int32).reshape(1, B) + torch.arange(1, steps + 1, dtype=torch.int32).reshape(-1, 1)
+        row = torch.arange(B, dtype=torch.int32).reshape(1, B).expand(steps, B)
+        host = torch.stack([torch.stack([lo, hi, hi - 1, torch.zeros_like(hi)], dim=-1),
+                            torch.stack([row, torch.ones_like(hi), lo, hi], dim=-1)])
+        self.qtab, self.tiles = host.to(device).unbind(0)
+        self.rows = (self.qtab[..., 1] - 1).long()
+        self.ktab = torch.zeros((k_rows, 4), dtype=torch.int32, device=device)  # no flagged keys: never read
+
+    def meta(self, i: int, rows_per_tile: int) -> AttnMeta:
+        m = copy.copy(self.base)
+        m.k_ranges = [(s, s + l + i + 1) for s, l in zip(self.starts, self.lens)]
+        m.cu_k_host = [r[0] for r in m.k_ranges] + [m.k_ranges[-1][1]]
+        m.max_k = max(self.lens) + i + 1
+        m.cache_rows = self.rows[i]
+        m._dev = {"tables": (self.qtab[i], self.ktab), ("tiles", rows_per_tile): self.tiles[i]}
+        return m
+
+
 def _attention_torch(q, k, v, meta: AttnMeta, hq, hkv, d, scale):
     """Per-sequence PyTorch evaluation (CPU oracle path)."""
     outs = []
@@ -796,23 +824,28 @@ def rope_cache_(qkv: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, cache_r
     return qkv
 
 
+def cached_attention_kind(meta: AttnMeta, rows: int, hq: int, hkv: int, d: int) -> int:
+    """Which kernel serves an inference call over cached keys: 2 csrc/attention_cached.cuh, 1 csrc/decode.cu, 0 the general
+    one."""
+    if 0 < meta.max_q <= CACHED_MAX_ROWS and _C().attn_cached_supported(hq, hkv, d):
+        return 2
+    return 1 if rows <= DECODE_MAX_ROWS and _C().attn_decode_supported(rows, hq, hkv, d) else 0
+
+
 def attention_decode(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, meta: AttnMeta, hq: int, hkv: int, d: int,
                      scale: Optional[float] = None) -> torch.Tensor:
     """:func:`attention` for a handful of query rows per sequence over a long cached key range (decode and denoise steps):
     the tensor-core kernel of csrc/attention_cached.cuh, or csrc/decode.cu where the heads of a group do not divide its
     128 rows. Inference only; falls back to :func:`attention` for shapes neither kernel serves."""
     scale = scale if scale is not None else 1.0 / math.sqrt(d)
-    if (_is_cuda(q) and not torch.is_grad_enabled() and 0 < meta.max_q <= CACHED_MAX_ROWS
-            and _C().attn_cached_supported(hq, hkv, d)):
-        qtab, ktab = meta.device_tables(q.device)
-        return _C().attn_cached(q, k, v, qtab, ktab, meta.row_tiles(q.device, 128 // (hq // hkv)), int(hq), int(hkv), int(d),
-                                float(scale), _attn_flags(meta)[0], int(meta.max_k))
-    if not (_is_cuda(q) and not torch.is_grad_enabled() and q.shape[0] <= DECODE_MAX_ROWS
-            and _C().attn_decode_supported(q.shape[0], hq, hkv, d)):
+    kind = cached_attention_kind(meta, q.shape[0], hq, hkv, d) if _is_cuda(q) and not torch.is_grad_enabled() else 0
+    if kind == 0:
         return attention(q, k, v, meta, hq, hkv, d, scale)
     qtab, ktab = meta.device_tables(q.device)
-    max_keys = max((k1 - k0 for k0, k1 in meta.k_ranges), default=0)
-    return _C().attn_decode(q, k, v, qtab, ktab, int(hq), int(hkv), int(d), float(scale), int(max_keys))
+    if kind == 2:
+        return _C().attn_cached(q, k, v, qtab, ktab, meta.row_tiles(q.device, 128 // (hq // hkv)), int(hq), int(hkv), int(d),
+                                float(scale), _attn_flags(meta)[0], int(meta.max_k))
+    return _C().attn_decode(q, k, v, qtab, ktab, int(hq), int(hkv), int(d), float(scale), int(meta.max_k))
 
 
 def attention_packed(qkv: torch.Tensor, meta: AttnMeta, hq: int, hkv: int, d: int,
