@@ -31,8 +31,6 @@
 // two products, the softmax and the merge.
 #pragma once
 
-#include "launch.h"
-
 #include <atomic>
 
 namespace wx {

@@ -552,6 +552,8 @@ gemm_kernel(const __grid_constant__ GemmArgs args, int* __restrict__ status) {
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = warp_uniform(*tmem_slot);
+  pdl_wait();
+  pdl_launch_dependents();
 
   Dims d;
   load_dims<BN>(args, d);
@@ -757,6 +759,7 @@ int launch_t(const GemmArgs& args, int grid, cudaStream_t stream, int* status) {
     if (e != cudaSuccess) return static_cast<int>(e);
     attr_set = true;
   }
+  if (!AG) return static_cast<int>(launch_kernel(kern, dim3(grid), dim3(kThreads), C::SMEM_BYTES, stream, args, status));
   kern<<<grid, kThreads, C::SMEM_BYTES, stream>>>(args, status);
   return static_cast<int>(cudaGetLastError());
 }

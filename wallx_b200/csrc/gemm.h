@@ -23,6 +23,7 @@ enum GemmFlags : int {
   // D2 (input) holds the saved raw gate/up values [*, 2N] in 16-column interleaved blocks and D
   // (output, bf16, 2N wide) receives dL/d(gate|up) in the same layout. N % 32 == 0.
   GEMM_SWIGLU_BWD = 32,
+  GEMM_B_FRESH = 64,     // B was written by the kernel launched just before: no load of it ahead of that kernel's end
 };
 
 struct GemmCall {

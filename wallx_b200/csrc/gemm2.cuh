@@ -84,6 +84,8 @@ gemm_pair_kernel(const __grid_constant__ GemmArgs args, int* __restrict__ status
   cluster_wait();
   tc_fence_after();
   const uint32_t tmem_base = warp_uniform(*tmem_slot);
+  pdl_wait();
+  pdl_launch_dependents();
 
   Dims d;
   load_dims<kPairTileN, kPairTileM>(args, d);
@@ -278,8 +280,8 @@ int launch_pair_t(const GemmArgs& args, long tiles, cudaStream_t stream, int* st
   const int cap = pair_capacity<A_MN, B_MN>();
   if (cap <= 0) return -10;
   const int pairs = tiles < cap ? static_cast<int>(tiles) : cap;
-  gemm_pair_kernel<A_MN, B_MN><<<2 * pairs, kThreads, kPairSmemBytes, stream>>>(args, status);
-  return static_cast<int>(cudaGetLastError());
+  return static_cast<int>(launch_kernel(gemm_pair_kernel<A_MN, B_MN, false>, dim3(2 * pairs), dim3(kThreads), kPairSmemBytes, stream,
+                                        args, status));
 }
 
 // Gathered-weight launch on CTA pairs: `n_pull` copy CTAs (even) + GEMM pairs; -10 when clusters cannot be scheduled

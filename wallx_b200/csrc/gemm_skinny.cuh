@@ -198,7 +198,7 @@ gemm_few_kernel(const __grid_constant__ GemmArgs args, int* __restrict__ status,
     fence_mbar_init();
     tma_prefetch_desc(&p.tmA);
     tma_prefetch_desc(&p.tmB);
-    if (p.dyn == nullptr && p.M > mt * nb && p.K > 0 && (p.k0 & 7) == 0 && n_base < p.N) {
+    if (p.dyn == nullptr && !(p.flags & GEMM_B_FRESH) && p.M > mt * nb && p.K > 0 && (p.k0 & 7) == 0 && n_base < p.N) {
       const int nkb_s = (p.K + BK - 1) / BK;
       const int b0 = static_cast<int>(static_cast<long>(nkb_s) * rank / splits);
       const int b1 = static_cast<int>(static_cast<long>(nkb_s) * (rank + 1) / splits);

@@ -52,7 +52,7 @@ std::tuple<at::Tensor, at::Tensor> rms_norm_bwd(const at::Tensor& dy, const at::
   const int T = x.size(0), C = x.size(1);
   at::Tensor dx = at::empty_like(x);
   at::Tensor dw = at::empty_like(w);
-  at::Tensor partial = at::empty({wx::rms_norm_bwd_blocks(T), C}, x.options().dtype(at::kFloat));
+  at::Tensor partial = at::empty({wx::rms_norm_bwd_blocks(T, C), C}, x.options().dtype(at::kFloat));
   WX_CHECK_RC(wx::rms_norm_bwd(dy.data_ptr(), x.data_ptr(), w.data_ptr(), rstd.data_ptr<float>(), opt_int(dest),
                                dx.data_ptr(), partial.data_ptr<float>(), dw.data_ptr(), T, C, cur_stream()),
               "rms_norm_bwd");

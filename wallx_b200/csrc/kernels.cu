@@ -232,92 +232,155 @@ rms_norm_fwd_warp_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat1
   }
 }
 
-template <int CH>
-__global__ void __launch_bounds__(256)
-rms_norm_bwd_warp_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
+// RMSNorm backward for C = 256 * n <= 2048: a row belongs to one warp (C < 1024) or to two (`PAIR`; half the registers per
+// lane, so that two blocks and not one sit on an SM), CH 16-byte pieces per lane, all loads of the row in flight at once,
+// the weight kept in registers. The block's eight warps add their weight-gradient sums pairwise (a fixed order) through
+// shared memory laid out without bank conflicts; one after the other, 8-way conflicted, that tail alone took 10 us.
+// 31104 x 1280: 90 us before, now 60; 11072 x 2048: 73 -> 55; 692 x 2048: 36 -> 9.5 (with the sum of the partials).
+constexpr int NORM_BWD_THREADS = 256;
+template <int CH, bool PAIR>
+__global__ void __launch_bounds__(NORM_BWD_THREADS, 2)
+rms_norm_bwd_rows_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
                          const __nv_bfloat16* __restrict__ w, const float* __restrict__ rstd_in,
                          const int* __restrict__ dest, __nv_bfloat16* __restrict__ dx, float* __restrict__ dw_partial,
-                         int T, const __nv_bfloat16* __restrict__ add) {
-  constexpr int C = CH * 256;
-  __shared__ float dws[C];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int i = threadIdx.x; i < C; i += 256) dws[i] = 0.f;
-  __syncthreads();
+                         int T, int C, const __nv_bfloat16* __restrict__ add) {
+  constexpr int LANES = PAIR ? 64 : 32;  // lanes of a row
+  constexpr int TEAMS = NORM_BWD_THREADS / LANES;
+  __shared__ float s_dw[TEAMS / 2][CH * 8][LANES];
+  __shared__ float s_dot[2][8];
+  const int lane = threadIdx.x & (LANES - 1), team = threadIdx.x / LANES, warp = threadIdx.x >> 5;
+  const int nchunk = C >> 3;
+  pdl_wait();
+  pdl_launch_dependents();
+  BF8 wraw[CH];
   float dwacc[CH][8];
 #pragma unroll
-  for (int c = 0; c < CH; ++c)
+  for (int c = 0; c < CH; ++c) {
+    if (lane + LANES * c < nchunk) wraw[c] = reinterpret_cast<const BF8*>(w)[lane + LANES * c];
 #pragma unroll
     for (int e = 0; e < 8; ++e) dwacc[c][e] = 0.f;
-  const BF8* wr = reinterpret_cast<const BF8*>(w);
-  for (int row = blockIdx.x * 8 + warp; row < T; row += gridDim.x * 8) {
+  }
+  const float inv_c = 1.f / static_cast<float>(C);
+  int parity = 0;
+  for (int row = blockIdx.x * TEAMS + team; row < T; row += gridDim.x * TEAMS, parity ^= 1) {
     const int grow = dest ? dest[row] : row;
     const BF8* xr = reinterpret_cast<const BF8*>(x + static_cast<size_t>(row) * C);
     const BF8* gr = reinterpret_cast<const BF8*>(dy + static_cast<size_t>(grow) * C);
+    const BF8* ar = add != nullptr ? reinterpret_cast<const BF8*>(add + static_cast<size_t>(row) * C) : nullptr;
     const float rstd = rstd_in[row];
     BF8 xraw[CH], graw[CH], araw[CH];
-    // all loads of the row are issued together (the residual-path gradient too: loading it after the reduction
-    // would put a second memory round trip on every row's critical path)
-    const BF8* ar = add != nullptr ? reinterpret_cast<const BF8*>(add + static_cast<size_t>(row) * C) : nullptr;
 #pragma unroll
     for (int c = 0; c < CH; ++c) {
-      xraw[c] = xr[lane + 32 * c];
-      graw[c] = gr[lane + 32 * c];
-      if (ar != nullptr) araw[c] = ar[lane + 32 * c];
+      const int i = lane + LANES * c;
+      if (i < nchunk) {
+        xraw[c] = xr[i];
+        graw[c] = gr[i];
+        if (ar != nullptr) araw[c] = ar[i];
+      }
     }
     float dot = 0.f;
 #pragma unroll
     for (int c = 0; c < CH; ++c) {
-      float xf[8], df[8], wf[8];
-      unpack8(xraw[c], xf);
-      unpack8(graw[c], df);
-      unpack8(wr[lane + 32 * c], wf);
+      if (lane + LANES * c < nchunk) {
+        float xf[8], df[8], wf[8];
+        unpack8(xraw[c], xf);
+        unpack8(graw[c], df);
+        unpack8(wraw[c], wf);
 #pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        const float xh = xf[e] * rstd;
-        dot += df[e] * wf[e] * xh;
-        dwacc[c][e] += df[e] * bf16_round(xh);
+        for (int e = 0; e < 8; ++e) {
+          const float xh = xf[e] * rstd;
+          dot += df[e] * wf[e] * xh;
+          dwacc[c][e] += df[e] * bf16_round(xh);
+        }
       }
     }
-    dot = warp_sum(dot) / static_cast<float>(C);
+    dot = warp_sum(dot);
+    if (PAIR) {
+      if ((threadIdx.x & 31) == 0) s_dot[parity][warp] = dot;
+      asm volatile("bar.sync %0, 64;" ::"r"(team + 1) : "memory");
+      dot = s_dot[parity][team * 2] + s_dot[parity][team * 2 + 1];
+    }
+    dot *= inv_c;
     BF8* dxr = reinterpret_cast<BF8*>(dx + static_cast<size_t>(row) * C);
 #pragma unroll
     for (int c = 0; c < CH; ++c) {
-      float xf[8], df[8], wf[8], o[8];
-      unpack8(xraw[c], xf);
-      unpack8(graw[c], df);
-      unpack8(wr[lane + 32 * c], wf);
+      const int i = lane + LANES * c;
+      if (i < nchunk) {
+        float xf[8], df[8], wf[8], o[8];
+        unpack8(xraw[c], xf);
+        unpack8(graw[c], df);
+        unpack8(wraw[c], wf);
 #pragma unroll
-      for (int e = 0; e < 8; ++e) o[e] = rstd * (df[e] * wf[e] - xf[e] * rstd * dot);
-      if (ar != nullptr) {  // + the gradient of the residual path, with the rounding of a separate bf16 add
-        float af[8];
-        unpack8(araw[c], af);
+        for (int e = 0; e < 8; ++e) o[e] = rstd * (df[e] * wf[e] - xf[e] * rstd * dot);
+        if (ar != nullptr) {  // + the gradient of the residual path, with the rounding of a separate bf16 add
+          float af[8];
+          unpack8(araw[c], af);
 #pragma unroll
-        for (int e = 0; e < 8; ++e) o[e] = bf16_round(o[e]) + af[e];
+          for (int e = 0; e < 8; ++e) o[e] = bf16_round(o[e]) + af[e];
+        }
+        dxr[i] = pack8(o);
       }
-      dxr[lane + 32 * c] = pack8(o);
     }
   }
-  // warps add their sums one after the other, so the result does not depend on timing
-  for (int wv = 0; wv < 8; ++wv) {
-    if (warp == wv) {
+#pragma unroll
+  for (int n = TEAMS / 2; n >= 1; n >>= 1) {
+    if (team >= n && team < 2 * n) {
 #pragma unroll
       for (int c = 0; c < CH; ++c)
 #pragma unroll
-        for (int e = 0; e < 8; ++e) dws[(lane + 32 * c) * 8 + e] += dwacc[c][e];
+        for (int e = 0; e < 8; ++e) s_dw[team - n][c * 8 + e][lane] = dwacc[c][e];
+    }
+    __syncthreads();
+    if (team < n) {
+#pragma unroll
+      for (int c = 0; c < CH; ++c)
+#pragma unroll
+        for (int e = 0; e < 8; ++e) dwacc[c][e] += s_dw[team][c * 8 + e][lane];
     }
     __syncthreads();
   }
-  float* dp = dw_partial + static_cast<size_t>(blockIdx.x) * C;
-  for (int i = threadIdx.x; i < C; i += 256) dp[i] = dws[i];
+  if (team == 0) {
+    float* dp = dw_partial + static_cast<size_t>(blockIdx.x) * C;
+#pragma unroll
+    for (int c = 0; c < CH; ++c) {
+      const int i = lane + LANES * c;
+      if (i < nchunk) {
+        *reinterpret_cast<float4*>(dp + i * 8) = make_float4(dwacc[c][0], dwacc[c][1], dwacc[c][2], dwacc[c][3]);
+        *reinterpret_cast<float4*>(dp + i * 8 + 4) = make_float4(dwacc[c][4], dwacc[c][5], dwacc[c][6], dwacc[c][7]);
+      }
+    }
+  }
 }
 
-__global__ void reduce_partials_kernel(const float* __restrict__ partial, __nv_bfloat16* __restrict__ out, int nblk,
-                                       int C) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= C) return;
+// out[c] = sum over `n` rows of part[., C], in a fixed order: eight warps take every eighth row of 32 columns (four loads in
+// flight each) and their sums are added in warp order. One thread per column walked all rows one load after the other:
+// 296 x 2048 took 11 us and 486 x 6912 34 us; the whole column sum of 31104 x 6912 went from 101 to 80 us.
+__global__ void __launch_bounds__(256)
+sum_rows_kernel(const float* __restrict__ part, __nv_bfloat16* __restrict__ out, int n, int C) {
+  __shared__ float red[8][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int c = blockIdx.x * 32 + lane;
+  pdl_wait();
+  pdl_launch_dependents();
   float s = 0.f;
-  for (int b = 0; b < nblk; ++b) s += partial[static_cast<size_t>(b) * C + c];
-  out[c] = __float2bfloat16(s);
+  if (c < C) {
+    int r = warp;
+    for (; r + 24 < n; r += 32) {
+      float v[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) v[u] = part[static_cast<size_t>(r + 8 * u) * C + c];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) s += v[u];
+    }
+    for (; r < n; r += 8) s += part[static_cast<size_t>(r) * C + c];
+  }
+  red[warp][lane] = s;
+  __syncthreads();
+  if (warp == 0 && c < C) {
+#pragma unroll
+    for (int w = 1; w < 8; ++w) s += red[w][lane];
+    out[c] = __float2bfloat16(s);
+  }
 }
 
 // ------------------------------------------------------------------------------ SwiGLU backward
@@ -362,6 +425,8 @@ rope_qk_kernel(const __nv_bfloat16* in, __nv_bfloat16* out, const float* __restr
   const int half = D >> 1;
   const int tpr = half >> 3;  // threads per token
   const long idx = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x;
+  pdl_wait();
+  pdl_launch_dependents();
   if (idx >= static_cast<long>(T) * tpr) return;
   const int t = static_cast<int>(idx / tpr);
   const int d0 = static_cast<int>(idx - static_cast<long>(t) * tpr) * 8;
@@ -413,6 +478,8 @@ __global__ void rope_qk_chunk_kernel(const __nv_bfloat16* in, __nv_bfloat16* out
   const int copy_chunks = copy_rest ? (W - n_rot * D) >> 3 : 0;
   const int per_row = rot_chunks + copy_chunks;
   const long idx = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x;
+  pdl_wait();
+  pdl_launch_dependents();
   if (idx >= static_cast<long>(T) * per_row) return;
   const int t = static_cast<int>(idx / per_row);
   const int c = static_cast<int>(idx - static_cast<long>(t) * per_row);
@@ -536,6 +603,8 @@ route_plan_kernel(const int* __restrict__ types, int T, int E, int rows, int* __
 __global__ void permute_rows_kernel(const __nv_bfloat16* __restrict__ x, const int* __restrict__ dest,
                                     __nv_bfloat16* __restrict__ out, int T, int C, int out_rows) {
   const int nchunk = C >> 3;
+  pdl_wait();
+  pdl_launch_dependents();
   for (int row = blockIdx.x; row < T; row += gridDim.x) {
     if (!WX_CHK(dest[row] >= 0 && (out_rows <= 0 || dest[row] < out_rows) && (C & 7) == 0, 4003, dest[row], out_rows)) continue;
     const BF8* src = reinterpret_cast<const BF8*>(x + static_cast<size_t>(row) * C);
@@ -562,6 +631,8 @@ __global__ void gather_rows_kernel(const __nv_bfloat16* __restrict__ x, const in
 __global__ void column_sum_kernel(const __nv_bfloat16* __restrict__ x, float* __restrict__ part, int R, int C,
                                   int rows_per_block) {
   const int c2 = blockIdx.x * blockDim.x + threadIdx.x;  // pair index
+  pdl_wait();
+  pdl_launch_dependents();
   if (c2 * 2 >= C) return;
   const int r0 = blockIdx.y * rows_per_block;
   const int r1 = min(R, r0 + rows_per_block);
@@ -588,6 +659,8 @@ __global__ void column_sum_kernel(const __nv_bfloat16* __restrict__ x, float* __
 __global__ void column_sum8_kernel(const __nv_bfloat16* __restrict__ x, float* __restrict__ part, int R, int C,
                                    int rows_per_block) {
   const int c8 = blockIdx.x * blockDim.x + threadIdx.x;
+  pdl_wait();
+  pdl_launch_dependents();
   if (c8 * 8 >= C) return;
   const int r0 = blockIdx.y * rows_per_block;
   const int r1 = min(R, r0 + rows_per_block);
@@ -615,14 +688,6 @@ __global__ void column_sum8_kernel(const __nv_bfloat16* __restrict__ x, float* _
   float* acc = part + static_cast<size_t>(blockIdx.y) * C + c8 * 8;
   *reinterpret_cast<float4*>(acc) = make_float4(s[0], s[1], s[2], s[3]);
   *reinterpret_cast<float4*>(acc + 4) = make_float4(s[4], s[5], s[6], s[7]);
-}
-__global__ void column_sum_finish_kernel(const float* __restrict__ part, __nv_bfloat16* __restrict__ out, int nslab,
-                                         int C) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= C) return;
-  float s = 0.f;
-  for (int y = 0; y < nslab; ++y) s += part[static_cast<size_t>(y) * C + c];
-  out[c] = __float2bfloat16(s);
 }
 __global__ void f32_to_bf16_kernel(const float* __restrict__ in, __nv_bfloat16* __restrict__ out, long n) {
   const long i = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -851,31 +916,45 @@ int rms_norm_fwd(const void* x, const void* w, void* y, float* rstd, const int* 
   return static_cast<int>(cudaGetLastError());
 }
 
-int rms_norm_bwd_blocks(int T) { return T < sm_count() * 2 ? (T > 0 ? T : 1) : sm_count() * 2; }
+namespace {
+bool norm_bwd_rows(int C) { return C % 256 == 0 && C <= 2048; }
+}  // namespace
+
+// Blocks of the backward kernel (rows of its weight-gradient partials): no more than have a row to work on.
+int rms_norm_bwd_blocks(int T, int C) {
+  const int per_block = !norm_bwd_rows(C) ? 1 : C >= 1024 ? 4 : 8;
+  const int need = (T + per_block - 1) / per_block;
+  const int most = sm_count() * 2;
+  return need < 1 ? 1 : need < most ? need : most;
+}
 
 int rms_norm_bwd(const void* dy, const void* x, const void* w, const float* rstd, const int* dest, void* dx,
                  float* dw_partial, void* dw, int T, int C, cudaStream_t s, const void* add) {
   const __nv_bfloat16* addb = reinterpret_cast<const __nv_bfloat16*>(add);
   if (C % 8 != 0 || C > NORM_THREADS * 8 * NORM_MAX_CHUNKS) return -1;
-  const int grid = rms_norm_bwd_blocks(T);
-  if (C % 256 == 0 && C <= 2048) {  // one warp per row; the number of partial rows is the same
-    const __nv_bfloat16* dyb = reinterpret_cast<const __nv_bfloat16*>(dy);
-    const __nv_bfloat16* xb = reinterpret_cast<const __nv_bfloat16*>(x);
-    const __nv_bfloat16* wb = reinterpret_cast<const __nv_bfloat16*>(w);
-    __nv_bfloat16* dxb = reinterpret_cast<__nv_bfloat16*>(dx);
-    switch (C / 256) {
-#define WX_CASE(n) case n: rms_norm_bwd_warp_kernel<n><<<grid, 256, 0, s>>>(dyb, xb, wb, rstd, dest, dxb, dw_partial, T, addb); break;
-      WX_CASE(1) WX_CASE(2) WX_CASE(3) WX_CASE(4) WX_CASE(5) WX_CASE(6) WX_CASE(7) WX_CASE(8)
-#undef WX_CASE
-    }
-    reduce_partials_kernel<<<(C + 255) / 256, 256, 0, s>>>(dw_partial, reinterpret_cast<__nv_bfloat16*>(dw), grid, C);
-    return static_cast<int>(cudaGetLastError());
+  const int grid = rms_norm_bwd_blocks(T, C);
+  const __nv_bfloat16* dyb = reinterpret_cast<const __nv_bfloat16*>(dy);
+  const __nv_bfloat16* xb = reinterpret_cast<const __nv_bfloat16*>(x);
+  const __nv_bfloat16* wb = reinterpret_cast<const __nv_bfloat16*>(w);
+  __nv_bfloat16* dxb = reinterpret_cast<__nv_bfloat16*>(dx);
+  cudaError_t e = cudaSuccess;
+  if (norm_bwd_rows(C)) {
+    auto run = [&](auto kern) {
+      return launch_kernel(kern, dim3(grid), dim3(NORM_BWD_THREADS), 0, s, dyb, xb, wb, rstd, dest, dxb, dw_partial, T, C, addb);
+    };
+    if (C == 256) e = run(rms_norm_bwd_rows_kernel<1, false>);
+    else if (C == 512) e = run(rms_norm_bwd_rows_kernel<2, false>);
+    else if (C == 768) e = run(rms_norm_bwd_rows_kernel<3, false>);
+    else if (C == 1024) e = run(rms_norm_bwd_rows_kernel<2, true>);
+    else if (C <= 1536) e = run(rms_norm_bwd_rows_kernel<3, true>);
+    else e = run(rms_norm_bwd_rows_kernel<4, true>);
+  } else {
+    rms_norm_bwd_kernel<<<grid, NORM_THREADS, 0, s>>>(dyb, xb, wb, rstd, dest, dxb, dw_partial, T, C, addb);
+    e = cudaGetLastError();
   }
-  rms_norm_bwd_kernel<<<grid, NORM_THREADS, 0, s>>>(
-      reinterpret_cast<const __nv_bfloat16*>(dy), reinterpret_cast<const __nv_bfloat16*>(x),
-      reinterpret_cast<const __nv_bfloat16*>(w), rstd, dest, reinterpret_cast<__nv_bfloat16*>(dx), dw_partial, T, C, addb);
-  reduce_partials_kernel<<<(C + 255) / 256, 256, 0, s>>>(dw_partial, reinterpret_cast<__nv_bfloat16*>(dw), grid, C);
-  return static_cast<int>(cudaGetLastError());
+  if (e == cudaSuccess)
+    e = launch_kernel(sum_rows_kernel, dim3((C + 31) / 32), dim3(256), 0, s, dw_partial, reinterpret_cast<__nv_bfloat16*>(dw), grid, C);
+  return static_cast<int>(e);
 }
 
 int swiglu_bwd(const void* dh, const void* gu, void* dgu, int R, int width_gu, long ld_dh, long ld_gu,
@@ -900,17 +979,15 @@ int rope_qk(const void* in, void* out, const float* cos_t, const float* sin_t, i
   // in place (in == out): every thread reads its rotation pairs before it writes them, and the columns that are not
   // rotated (v) need no copy, which saves a third of the traffic of a q|k|v buffer with as many v as q heads
   const int copy_rest = (in != out) ? 1 : 0;
+  const __nv_bfloat16* src = reinterpret_cast<const __nv_bfloat16*>(in);
+  __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(out);
   if (total < static_cast<long>(sm_count()) * 256 || D % 128 != 0) {
     const long per_row = static_cast<long>(n_rot) * (D / 16) + (copy_rest ? (W - n_rot * D) / 8 : 0);
-    rope_qk_chunk_kernel<<<static_cast<unsigned>((per_row * T + 255) / 256), 256, 0, s>>>(
-        reinterpret_cast<const __nv_bfloat16*>(in), reinterpret_cast<__nv_bfloat16*>(out), cos_t, sin_t, T, W, n_rot, D,
-        inverse, copy_rest);
-    return static_cast<int>(cudaGetLastError());
+    return static_cast<int>(launch_kernel(rope_qk_chunk_kernel, dim3(static_cast<unsigned>((per_row * T + 255) / 256)), dim3(256), 0, s,
+                                          src, dst, cos_t, sin_t, T, W, n_rot, D, inverse, copy_rest));
   }
-  rope_qk_kernel<<<static_cast<unsigned>((total + 255) / 256), 256, 0, s>>>(
-      reinterpret_cast<const __nv_bfloat16*>(in), reinterpret_cast<__nv_bfloat16*>(out), cos_t, sin_t, T, W, n_rot, D,
-      inverse, copy_rest);
-  return static_cast<int>(cudaGetLastError());
+  return static_cast<int>(launch_kernel(rope_qk_kernel, dim3(static_cast<unsigned>((total + 255) / 256)), dim3(256), 0, s, src, dst,
+                                        cos_t, sin_t, T, W, n_rot, D, inverse, copy_rest));
 }
 
 int route_plan(const int* types, int T, int E, int rows, int* dest, int* seg, int* segk, int* inv, cudaStream_t s) {
@@ -922,9 +999,9 @@ int route_plan(const int* types, int T, int E, int rows, int* dest, int* seg, in
 int permute_rows(const void* x, const int* dest, void* out, int T, int C, cudaStream_t s, int out_rows) {
   if (C % 8 != 0) return -1;
   if (T == 0) return 0;
-  permute_rows_kernel<<<T < sm_count() * 16 ? T : sm_count() * 16, 128, 0, s>>>(reinterpret_cast<const __nv_bfloat16*>(x), dest,
-                                                                  reinterpret_cast<__nv_bfloat16*>(out), T, C, out_rows);
-  return static_cast<int>(cudaGetLastError());
+  return static_cast<int>(launch_kernel(permute_rows_kernel, dim3(T < sm_count() * 16 ? T : sm_count() * 16), dim3(128), 0, s,
+                                        reinterpret_cast<const __nv_bfloat16*>(x), dest, reinterpret_cast<__nv_bfloat16*>(out), T, C,
+                                        out_rows));
 }
 
 int gather_rows(const void* x, const int* idx, void* out, int T, int C, cudaStream_t s, int src_rows) {
@@ -947,15 +1024,15 @@ int column_sum(const void* x, float* partials, void* out_bf16, int R, int C, cud
   const int pairs = (C + 1) / 2;
   const int ysplit = column_sum_slabs(R);
   const int rpb = (R + ysplit - 1) / ysplit;
-  if (C % 8 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0) {
-    dim3 grid8((C / 8 + 63) / 64, ysplit);
-    column_sum8_kernel<<<grid8, 64, 0, s>>>(reinterpret_cast<const __nv_bfloat16*>(x), partials, R, C, rpb);
-  } else {
-    dim3 grid((pairs + 127) / 128, ysplit);
-    column_sum_kernel<<<grid, 128, 0, s>>>(reinterpret_cast<const __nv_bfloat16*>(x), partials, R, C, rpb);
-  }
-  column_sum_finish_kernel<<<(C + 255) / 256, 256, 0, s>>>(partials, reinterpret_cast<__nv_bfloat16*>(out_bf16), ysplit, C);
-  return static_cast<int>(cudaGetLastError());
+  const __nv_bfloat16* xb = reinterpret_cast<const __nv_bfloat16*>(x);
+  cudaError_t e;
+  if (C % 8 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0)
+    e = launch_kernel(column_sum8_kernel, dim3((C / 8 + 63) / 64, ysplit), dim3(64), 0, s, xb, partials, R, C, rpb);
+  else
+    e = launch_kernel(column_sum_kernel, dim3((pairs + 127) / 128, ysplit), dim3(128), 0, s, xb, partials, R, C, rpb);
+  if (e == cudaSuccess)
+    e = launch_kernel(sum_rows_kernel, dim3((C + 31) / 32), dim3(256), 0, s, partials, reinterpret_cast<__nv_bfloat16*>(out_bf16), ysplit, C);
+  return static_cast<int>(e);
 }
 
 int ce_fwd(const void* logits, const long* labels, float* loss, float* lse, long* pred, int R, int V, long ld,

@@ -11,7 +11,7 @@ namespace wx {
 
 int rms_norm_fwd(const void* x, const void* w, void* y, float* rstd, const int* dest, int T, int C, float eps,
                  cudaStream_t s);
-int rms_norm_bwd_blocks(int T);
+int rms_norm_bwd_blocks(int T, int C);
 // `add` (optional, bf16 [T, C]): added to dx with the rounding of a separate bf16 add (the gradient that arrives
 // over the residual connection around the normalised branch).
 int rms_norm_bwd(const void* dy, const void* x, const void* w, const float* rstd, const int* dest, void* dx,

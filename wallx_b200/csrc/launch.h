@@ -6,8 +6,9 @@
 // are visible. Every kernel launched this way therefore calls pdl_wait() before its first access to global memory
 // that an earlier kernel may have written, and pdl_launch_dependents() once the next kernel may begin its own
 // prologue. Both instructions do nothing in a kernel that was launched the ordinary way, and a kernel without
-// pdl_wait() is never launched through this helper. The switch is off by default (training launches are unchanged);
-// the flow engine turns it on around its graph capture.
+// pdl_wait() is never launched through this helper. The switch belongs to the calling thread and is off by default;
+// inference entry points turn it on for their whole call, and the whole-block entry points (csrc/blocks.cpp) around the
+// kernels of one block.
 #pragma once
 #include <cuda_runtime.h>
 

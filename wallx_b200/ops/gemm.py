@@ -23,6 +23,7 @@ ACCUMULATE = 2
 ACT_GELU = 4
 ACT_SWIGLU = 8
 ZERO_PAD_ROWS = 16
+B_FRESH = 64  # the B operand was written by the kernel launched just before: no load of it ahead of that kernel's end
 SWIGLU_BWD = 32  # accumulator = dL/dh; out2 = saved raw gate/up (input); out = dL/d(gate|up), 2N wide
 
 
