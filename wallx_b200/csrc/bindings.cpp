@@ -88,6 +88,7 @@ void fill_call(wx::GemmCall& c, const GemmTuple& g) {
   c.residual = opt_ptr(residual);
   c.ldr = c.residual ? residual->stride(0) : 0;
   if (c.residual) TORCH_CHECK(residual->scalar_type() == at::kBFloat16 && residual->stride(1) == 1, "gemm: residual");
+  c.qkv = nullptr;
   c.row_map = reinterpret_cast<const int*>(opt_ptr(row_map));
   if (c.row_map) TORCH_CHECK(row_map->scalar_type() == at::kInt, "gemm: row_map int32");
   c.dyn = reinterpret_cast<const int*>(opt_ptr(dyn));

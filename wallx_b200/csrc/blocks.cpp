@@ -72,9 +72,10 @@ wxb::GemmTuple to_tuple(const Spec& s) {
                         0, 0);
 }
 
-void launch_plain(const Spec* specs, int n, int* status, int force_bn = 0) {
+void launch_plain(const Spec* specs, int n, int* status, int force_bn = 0, wx::QkvCache* qkv = nullptr) {
   wx::GemmCall cs[2];
   for (int i = 0; i < n; ++i) wxb::fill_call(cs[i], to_tuple(specs[i]));
+  cs[0].qkv = qkv;
   WX_RC(wx::gemm_launch(cs, n, cur(), status, force_bn), "gemm_launch");
 }
 
@@ -422,11 +423,15 @@ c10::optional<Tensor> block_cached(const Tensor& x, const Tensor& ln1_w, const T
     s.b = w_qkv;
     s.out = qkv;
     s.bias = b_qkv;
-    launch_plain(&s, 1, status, force);
+    // the few-row GEMM rotates and writes the cache in its epilogue; the general one leaves that to a kernel of its own
+    wx::QkvCache qc{cos_t.data_ptr<float>(), sin_t.data_ptr<float>(), cache_rows.data_ptr<int64_t>(), cache.data_ptr(),
+                    cache.stride(0), cache.size(0), static_cast<int>(hq), static_cast<int>(hkv), false};
+    launch_plain(&s, 1, status, force, d == 128 ? &qc : nullptr);
+    if (!qc.done)
+      WX_RC(wx::rope_cache(qkv.data_ptr(), qc.cos_t, qc.sin_t, qc.rows, cache.data_ptr(), T, W, hq, hkv, d, cache.stride(0),
+                           cache.size(0), cur()),
+            "rope_cache");
   }
-  WX_RC(wx::rope_cache(qkv.data_ptr(), cos_t.data_ptr<float>(), sin_t.data_ptr<float>(), cache_rows.data_ptr<int64_t>(),
-                       cache.data_ptr(), T, W, hq, hkv, d, cache.stride(0), cache.size(0), cur()),
-        "rope_cache");
   Tensor o = empty_bf16(T, hq * d, x);
   {
     Tensor k = cache.narrow(1, 0, hkv * d), v = cache.narrow(1, hkv * d, hkv * d);

@@ -79,8 +79,10 @@ rope_cache_kernel(__nv_bfloat16* qkv, const float* __restrict__ cos_t, const flo
   for (int e = 0; e < 4; ++e) {
     const float2 a = __bfloat1622float2(pa.v[e]);
     const float2 b = __bfloat1622float2(pb.v[e]);
-    oa.v[e] = __floats2bfloat162_rn(a.x * c1[2 * e] - b.x * s1[2 * e], a.y * c1[2 * e + 1] - b.y * s1[2 * e + 1]);
-    ob.v[e] = __floats2bfloat162_rn(b.x * c2[2 * e] + a.x * s2[2 * e], b.y * c2[2 * e + 1] + a.y * s2[2 * e + 1]);
+    oa.v[e] = __floats2bfloat162_rn(fmaf(a.x, c1[2 * e], -__fmul_rn(b.x, s1[2 * e])),
+                                    fmaf(a.y, c1[2 * e + 1], -__fmul_rn(b.y, s1[2 * e + 1])));
+    ob.v[e] = __floats2bfloat162_rn(fmaf(b.x, c2[2 * e], __fmul_rn(a.x, s2[2 * e])),
+                                    fmaf(b.y, c2[2 * e + 1], __fmul_rn(a.y, s2[2 * e + 1])));
   }
   __nv_bfloat16* dst = (h < hq) ? row + h * D : dst_row + (h - hq) * D;  // q in place, k to its cache slot
   *reinterpret_cast<Pack8*>(dst + d0) = oa;

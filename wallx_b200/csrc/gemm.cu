@@ -43,6 +43,13 @@ struct Problem {
   const int* dyn;
   long ldd, ldd2, ldr, d_rows;
   int M, N, K, m0, k0, flags;
+  // few-row kernel with kFewQkvCache: see QkvCache
+  const float* cos_t;
+  const float* sin_t;
+  const long* cache_rows;
+  __nv_bfloat16* cache;
+  long ld_cache, cache_nrows;
+  int q_tiles, kv_tiles;  // heads of q, heads of k (and of v)
 };
 
 // Device view of a fused weight gather (see AgInfo). The weight is one run of `total_bytes`

@@ -26,6 +26,19 @@ enum GemmFlags : int {
   GEMM_B_FRESH = 64,     // B was written by the kernel launched just before: no load of it ahead of that kernel's end
 };
 
+// Rotary and key-value cache write behind a q|k|v projection (heads of 128, q heads, then k, then v; no other epilogue but
+// the bias): row r's q heads are rotated and stored to D, its k heads rotated and its v heads plain to row rows[r] of
+// `cache` (k then v). A launch that did so sets `done`; otherwise D holds the plain projection (csrc/decode.h follows).
+struct QkvCache {
+  const float* cos_t;  // fp32 [M, 128]
+  const float* sin_t;
+  const long* rows;
+  void* cache;
+  long ld_cache, cache_nrows;
+  int hq, hkv;
+  bool done;
+};
+
 struct GemmCall {
   // A(m, k): a_mn == false -> memory [a_rows][>=k0+K], k contiguous, pitch lda elements.
   //          a_mn == true  -> memory [k rows][a_rows'], m contiguous, pitch lda elements.
@@ -55,6 +68,7 @@ struct GemmCall {
   long ldr;
   const int* row_map;  // optional: D row r is written to row row_map[r]; negative -> dropped
   int flags;
+  QkvCache* qkv;  // optional
 };
 
 // Weight all-gather fused into the GEMM (ZeRO-3 style sharded weight): B's rows are split evenly

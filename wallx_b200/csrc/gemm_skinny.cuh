@@ -37,6 +37,7 @@ constexpr int kFewWarps = kFewThreads / 32;
 constexpr int kFewMaxRows = 256;       // activation rows per tile: the N of an MMA
 constexpr int kFewMaxSplits = 8;       // portable cluster size
 constexpr int kFewBBytes = kFewBN * BK * 2;
+constexpr int kFewQkvCache = 1 << 16;  // internal flag of a problem: rotary and cache write in the epilogue
 
 struct FewShape {
   int nb;      // activation rows per tile: a multiple of 16
@@ -62,6 +63,37 @@ __device__ __forceinline__ void epilogue_quad(const Problem& p, float4 acc, long
 #pragma unroll
     for (int j = 0; j < 4; ++j)
       if (j < nvalid) v[j] += __bfloat162float(p.bias[n + j]);
+  }
+  if (flags & kFewQkvCache) {
+    // a tile is one head; rotation pairs are 64 columns apart, so sixteen lanes. The projection is rounded to bf16 first and
+    // the products are those of rope_cache_kernel.
+    const int head = n >> 7, d = n & 127;
+    const float4 x = bf16x4_to_f32(make_uint2(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3])));
+    float4 y;
+    y.x = __shfl_xor_sync(0xffffffffu, x.x, 16);
+    y.y = __shfl_xor_sync(0xffffffffu, x.y, 16);
+    y.z = __shfl_xor_sync(0xffffffffu, x.z, 16);
+    y.w = __shfl_xor_sync(0xffffffffu, x.w, 16);
+    float4 o = x;
+    if (head < p.q_tiles + p.kv_tiles) {
+      const float4 c = *reinterpret_cast<const float4*>(p.cos_t + drow * 128 + d);
+      float4 s = *reinterpret_cast<const float4*>(p.sin_t + drow * 128 + d);
+      if (d < 64) s = make_float4(-s.x, -s.y, -s.z, -s.w);
+      o.x = fmaf(x.x, c.x, __fmul_rn(y.x, s.x));
+      o.y = fmaf(x.y, c.y, __fmul_rn(y.y, s.y));
+      o.z = fmaf(x.z, c.z, __fmul_rn(y.z, s.z));
+      o.w = fmaf(x.w, c.w, __fmul_rn(y.w, s.w));
+    }
+    __nv_bfloat16* dst;
+    if (head < p.q_tiles) {
+      dst = reinterpret_cast<__nv_bfloat16*>(p.D) + drow * p.ldd + n;
+    } else {
+      const long crow = p.cache_rows[drow];
+      if (!WX_CHK(crow >= 0 && crow < p.cache_nrows, 2008, crow, p.cache_nrows)) return;
+      dst = p.cache + crow * p.ld_cache + (n - p.q_tiles * 128);
+    }
+    *reinterpret_cast<uint2*>(dst) = make_uint2(pack_bf16x2(o.x, o.y), pack_bf16x2(o.z, o.w));
+    return;
   }
   if (flags & GEMM_SWIGLU_BWD) {  // v = dL/dh of channels [n, n + 4); N is a multiple of 32
     if (nvalid <= 0) return;
@@ -383,7 +415,7 @@ gemm_few_kernel(const __grid_constant__ GemmArgs args, int* __restrict__ status,
 }
 
 constexpr int kFewSmemMax = 227 * 1024;
-constexpr int kFewSmemHalf = 113 * 1024;  // two CTAs of this size share an SM
+constexpr int kFewSmemHalf = 112 * 1024;  // two CTAs of this size (and 1 KB each that the system takes) share an SM
 constexpr int kFewSmemExtra = 1024 + 512;
 
 inline int few_smem(const FewShape& sh) { return sh.stages * (kFewBBytes + sh.nb * BK * 2) + kFewSmemExtra; }
@@ -448,6 +480,26 @@ int launch_few(const GemmCall* calls, int ncalls, const FewShape& sh, cudaStream
   GemmArgs args;
   const int rc = fill_args(args, calls, ncalls, kFewBN, sh.nb);
   if (rc != 0) return rc;
+  QkvCache* qc = calls[0].qkv;
+  if (qc != nullptr) {
+    const GemmCall& c = calls[0];
+    const auto aligned = [](const void* q, int bytes) { return (reinterpret_cast<uintptr_t>(q) & (bytes - 1)) == 0; };
+    if (ncalls == 1 && c.flags == 0 && c.row_map == nullptr && c.dyn == nullptr && c.residual == nullptr && c.m0 == 0 &&
+        c.N == (qc->hq + 2 * qc->hkv) * 128 && (c.ldd & 3) == 0 && aligned(c.D, 8) && (qc->ld_cache & 3) == 0 &&
+        aligned(qc->cache, 8) && aligned(qc->cos_t, 16) && aligned(qc->sin_t, 16)) {
+      Problem& p = args.p[0];
+      p.flags |= kFewQkvCache;
+      p.cos_t = qc->cos_t;
+      p.sin_t = qc->sin_t;
+      p.cache_rows = qc->rows;
+      p.cache = reinterpret_cast<__nv_bfloat16*>(qc->cache);
+      p.ld_cache = qc->ld_cache;
+      p.cache_nrows = qc->cache_nrows;
+      p.q_tiles = qc->hq;
+      p.kv_tiles = qc->hkv;
+      qc->done = true;
+    }
+  }
   long tiles = 0;
   for (int i = 0; i < ncalls; ++i)
     tiles += static_cast<long>((calls[i].N + kFewBN - 1) / kFewBN) * ((calls[i].M + sh.nb - 1) / sh.nb);

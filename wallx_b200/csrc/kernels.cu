@@ -450,11 +450,11 @@ rope_qk_kernel(const __nv_bfloat16* in, __nv_bfloat16* out, const float* __restr
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
       if (!inverse) {
-        oa[e] = a[e] * c1[e] - b[e] * s1[e];
-        ob[e] = b[e] * c2[e] + a[e] * s2[e];
+        oa[e] = fmaf(a[e], c1[e], -__fmul_rn(b[e], s1[e]));
+        ob[e] = fmaf(b[e], c2[e], __fmul_rn(a[e], s2[e]));
       } else {
-        oa[e] = a[e] * c1[e] + b[e] * s2[e];
-        ob[e] = b[e] * c2[e] - a[e] * s1[e];
+        oa[e] = fmaf(a[e], c1[e], __fmul_rn(b[e], s2[e]));
+        ob[e] = fmaf(b[e], c2[e], -__fmul_rn(a[e], s1[e]));
       }
     }
     *reinterpret_cast<BF8*>(orow + h * D + d0) = pack8(oa);
@@ -508,11 +508,11 @@ __global__ void rope_qk_chunk_kernel(const __nv_bfloat16* in, __nv_bfloat16* out
 #pragma unroll
   for (int e = 0; e < 8; ++e) {
     if (!inverse) {
-      oa[e] = a[e] * c1[e] - b[e] * s1[e];
-      ob[e] = b[e] * c2[e] + a[e] * s2[e];
+      oa[e] = fmaf(a[e], c1[e], -__fmul_rn(b[e], s1[e]));
+      ob[e] = fmaf(b[e], c2[e], __fmul_rn(a[e], s2[e]));
     } else {
-      oa[e] = a[e] * c1[e] + b[e] * s2[e];
-      ob[e] = b[e] * c2[e] - a[e] * s1[e];
+      oa[e] = fmaf(a[e], c1[e], __fmul_rn(b[e], s2[e]));
+      ob[e] = fmaf(b[e], c2[e], -__fmul_rn(a[e], s1[e]));
     }
   }
   *reinterpret_cast<BF8*>(orow + h * D + d0) = pack8(oa);
