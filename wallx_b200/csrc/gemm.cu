@@ -35,6 +35,9 @@ constexpr int kEpiWarp0 = 2;
 struct Problem {
   CUtensorMap tmA;
   CUtensorMap tmB;
+  CUtensorMap tmD;   // tma_out: D as boxes of 32 rows x 32 columns (SwiGLU: 16; its backward: 64)
+  CUtensorMap tmD2;  // tma_out with raw SwiGLU values: D2 as boxes of 32 x 32 (backward, read: 32 x 64)
+  int tma_out;
   void* D;
   void* D2;
   const __nv_bfloat16* bias;
@@ -82,6 +85,10 @@ constexpr int kAgDepth = kAgRing - 2;  // loads in flight
 constexpr int kAgLag = 3;               // store groups that may still be in flight behind a published tile
 constexpr int kAgPend = 8;              // tiles waiting for their stores' completion (power of two)
 
+constexpr int kEpiWarpStage = 4096;                    // staging of an epilogue warp: two chunks of 32 rows x 64 bytes
+constexpr int kEpiStage = kEpiWarps * kEpiWarpStage;
+constexpr int kEpiBarBytes = kEpiWarps * 2 * 8;  // two barriers per epilogue warp, 256 bytes behind the staging area
+
 template <int BN>
 struct Cfg {
   static constexpr int A_BYTES = BM * BK * 2;
@@ -89,7 +96,8 @@ struct Cfg {
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
   static constexpr int STAGES = (BN == 256) ? 4 : (BN == 128) ? 6 : 8;
   static constexpr int TMEM_COLS = (2 * BN < 32) ? 32 : 2 * BN;
-  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 256;
+  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + kEpiStage + 1024 + 256 + kEpiBarBytes;
+  static_assert(SMEM_BYTES <= 227 * 1024 && (STAGES * STAGE_BYTES) % 1024 == 0, "stages and epilogue staging must fit");
 };
 
 constexpr int kRasterGroup = 8;
@@ -326,9 +334,205 @@ __device__ __forceinline__ void epilogue_chunk(const Problem& p, float (&v)[32],
 // quarter, BN fp32 columns starting at taddr0) go through bias / activation / residual / row map /
 // accumulate and are stored. `row_in_prob` is this thread's row within the problem; the warp
 // handles the 32-column chunks [chunk0, chunk1) (two warps share a lane quarter).
+// Epilogue of a warp whose 32 rows all exist and whose output is bf16 without a row map: the rows of a chunk are staged in
+// shared memory and leave as one bulk tensor store, and what is read in place (gradients that are added to, saved raw
+// gate / up values) arrives as one bulk tensor load. A row per thread accessed 16 bytes of each of 32 lines per instruction,
+// which bounded every tile with a short K (us, before -> now):
+//   31104 x 3840 x 1280, bias 312 -> 252            10048 x 22016 x 2048, SwiGLU + raw 835 -> 753
+//   31104 x 3456 x 1280, SwiGLU backward 529 -> 445   10048 x 11008 x 2048, SwiGLU backward 649 -> 538
+//   22016 x 2048 x 692, plain 82 -> 65, adding 114 -> 85
+template <int BN>
+__device__ __forceinline__ void epilogue_rows_tma(const Problem& p, int drow, int lane, int n_base, uint32_t taddr0, int chunk0,
+                                                  int chunk1, uint8_t* stage, uint64_t* bar, uint32_t& phase,
+                                                  volatile int* abort_flag) {
+  const bool swiglu = (p.flags & GEMM_ACT_SWIGLU) != 0, accum = (p.flags & GEMM_ACCUMULATE) != 0;
+  if (chunk0 < chunk1 && n_base + (chunk1 - 1) * 32 >= p.N) chunk1 = max(chunk0, (p.N - n_base + 31) / 32);
+  if (chunk0 >= chunk1) return;
+  if (p.flags & GEMM_SWIGLU_BWD) {
+    // the saved raw values of 32 channels (two blocks of [16 gate | 16 up]) come in as one box, are replaced by their
+    // gradients and leave the same way
+    auto fetch = [&](int c) {
+      mbar_arrive_expect_tx(bar, 4096u);
+      tma_load_2d(stage, &p.tmD2, bar, 2 * (n_base + c * 32), drow);
+    };
+    if (lane == 0) {
+      bulk_store_wait_read<0>();
+      fetch(chunk0);
+    }
+#pragma unroll 1
+    for (int c = chunk0; c < chunk1; ++c) {
+      uint32_t r[32];
+      tmem_ld_32x32(taddr0 + c * 32, r);
+      tmem_ld_wait();
+      if (!mbar_wait(bar, phase & 1u, abort_flag)) return;
+      phase ^= 1u;
+#pragma unroll
+      for (int blk = 0; blk < 2; ++blk) {
+        uint4 raw[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) raw[q] = *reinterpret_cast<const uint4*>(stage + sw128_offset(lane, 4 * blk + q));
+        const __nv_bfloat162* gb = reinterpret_cast<const __nv_bfloat162*>(&raw[0]);  // 16 gate values
+        const __nv_bfloat162* ub = reinterpret_cast<const __nv_bfloat162*>(&raw[2]);  // 16 up values
+        uint32_t og[8], ou[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          const float2 g2 = __bfloat1622float2(gb[e]);
+          const float2 u2 = __bfloat1622float2(ub[e]);
+          const float d0 = __uint_as_float(r[16 * blk + 2 * e]), d1 = __uint_as_float(r[16 * blk + 2 * e + 1]);
+          const float s0 = 1.0f / (1.0f + __expf(-g2.x)), s1 = 1.0f / (1.0f + __expf(-g2.y));
+          og[e] = pack_bf16x2(d0 * u2.x * s0 * (1.0f + g2.x * (1.0f - s0)), d1 * u2.y * s1 * (1.0f + g2.y * (1.0f - s1)));
+          ou[e] = pack_bf16x2(d0 * g2.x * s0, d1 * g2.y * s1);
+        }
+        *reinterpret_cast<uint4*>(stage + sw128_offset(lane, 4 * blk + 0)) = make_uint4(og[0], og[1], og[2], og[3]);
+        *reinterpret_cast<uint4*>(stage + sw128_offset(lane, 4 * blk + 1)) = make_uint4(og[4], og[5], og[6], og[7]);
+        *reinterpret_cast<uint4*>(stage + sw128_offset(lane, 4 * blk + 2)) = make_uint4(ou[0], ou[1], ou[2], ou[3]);
+        *reinterpret_cast<uint4*>(stage + sw128_offset(lane, 4 * blk + 3)) = make_uint4(ou[4], ou[5], ou[6], ou[7]);
+      }
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) {
+        tma_store_2d(&p.tmD, stage, 2 * (n_base + c * 32), drow);
+        tma_store_commit();
+        if (c + 1 < chunk1) {
+          bulk_store_wait_read<0>();
+          fetch(c + 1);
+        }
+      }
+    }
+    return;
+  }
+  // old values that are added to: requested two chunks ahead, replaced in place
+  auto fetch = [&](int c) {
+    const int b = (c - chunk0) & 1;
+    mbar_arrive_expect_tx(&bar[b], 2048u);
+    tma_load_2d(stage + b * 2048, &p.tmD, &bar[b], n_base + c * 32, drow);
+  };
+  const bool res_vec = (p.ldr & 7) == 0 && (reinterpret_cast<uintptr_t>(p.residual) & 15) == 0;
+  const uint32_t swz = static_cast<uint32_t>(lane >> 1) & 3u;  // 64-byte swizzle: 16-byte piece ^ (row / 2) % 4
+  const __nv_bfloat16* rrow = p.residual != nullptr ? p.residual + static_cast<long>(drow + lane) * p.ldr : nullptr;
+  if (lane == 0) {
+    bulk_store_wait_read<0>();  // the previous tile's stores have read the staging area (long ago)
+    if (accum) {
+      fetch(chunk0);
+      if (chunk0 + 1 < chunk1) fetch(chunk0 + 1);
+    }
+  }
+#pragma unroll 1
+  for (int c = chunk0; c < chunk1; ++c) {
+    const int n0 = n_base + c * 32;
+    const int nvalid = min(32, p.N - n0);
+    uint32_t r[32];
+    tmem_ld_32x32(taddr0 + c * 32, r);
+    uint4 res[4];
+    const bool res_now = rrow != nullptr && nvalid == 32 && res_vec;
+    if (res_now) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) res[q] = reinterpret_cast<const uint4*>(rrow + n0)[q];
+    }
+    tmem_ld_wait();
+    float v[32];
+#pragma unroll
+    for (int e = 0; e < 32; ++e) v[e] = __uint_as_float(r[e]);
+    if (p.bias != nullptr) {
+#pragma unroll
+      for (int e = 0; e < 32; ++e)
+        if (e < nvalid) v[e] += __bfloat162float(p.bias[n0 + e]);
+    }
+    uint8_t* buf = stage;
+    if (swiglu) {
+      if (lane == 0) bulk_store_wait_read<0>();
+    } else {
+      const int b = (c - chunk0) & 1;
+      buf += b * 2048;
+      if (!accum && lane == 0) bulk_store_wait_read<1>();
+      if (p.flags & GEMM_ACT_GELU) {
+#pragma unroll
+        for (int e = 0; e < 32; ++e) v[e] = gelu_erf(v[e]);
+      }
+      if (res_now) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const __nv_bfloat162* xb = reinterpret_cast<const __nv_bfloat162*>(&res[q]);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float2 f = __bfloat1622float2(xb[e]);
+            v[8 * q + 2 * e] += f.x;
+            v[8 * q + 2 * e + 1] += f.y;
+          }
+        }
+      } else if (rrow != nullptr) {
+#pragma unroll
+        for (int e = 0; e < 32; ++e)
+          if (e < nvalid) v[e] += __bfloat162float(rrow[n0 + e]);
+      }
+      if (accum) {
+        if (!mbar_wait(&bar[b], (phase >> b) & 1u, abort_flag)) return;
+        phase ^= 1u << b;
+#pragma unroll
+        for (uint32_t q = 0; q < 4; ++q) {
+          const uint4 x = *reinterpret_cast<const uint4*>(buf + lane * 64 + ((q ^ swz) << 4));
+          const __nv_bfloat162* xb = reinterpret_cast<const __nv_bfloat162*>(&x);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float2 f = __bfloat1622float2(xb[e]);
+            v[8 * q + 2 * e] += f.x;
+            v[8 * q + 2 * e + 1] += f.y;
+          }
+        }
+      }
+    }
+    __syncwarp();
+    if (!swiglu || p.D2 != nullptr) {
+#pragma unroll
+      for (uint32_t q = 0; q < 4; ++q)
+        *reinterpret_cast<uint4*>(buf + lane * 64 + ((q ^ swz) << 4)) =
+            make_uint4(pack_bf16x2(v[8 * q + 0], v[8 * q + 1]), pack_bf16x2(v[8 * q + 2], v[8 * q + 3]),
+                       pack_bf16x2(v[8 * q + 4], v[8 * q + 5]), pack_bf16x2(v[8 * q + 6], v[8 * q + 7]));
+    }
+    if (swiglu) {  // columns [n0, n0 + 16) are gate, the next 16 up; rounded to bf16 first as in the unfused path
+      float h[16];
+#pragma unroll
+      for (int e = 0; e < 16; ++e)
+        h[e] = silu_f(__bfloat162float(__float2bfloat16(v[e]))) * __bfloat162float(__float2bfloat16(v[16 + e]));
+#pragma unroll
+      for (int q = 0; q < 2; ++q)
+        *reinterpret_cast<uint4*>(buf + 2048 + lane * 32 + q * 16) =
+            make_uint4(pack_bf16x2(h[8 * q + 0], h[8 * q + 1]), pack_bf16x2(h[8 * q + 2], h[8 * q + 3]),
+                       pack_bf16x2(h[8 * q + 4], h[8 * q + 5]), pack_bf16x2(h[8 * q + 6], h[8 * q + 7]));
+    }
+    fence_proxy_async_smem();
+    __syncwarp();
+    if (lane == 0) {
+      if (swiglu) {
+        if (p.D2 != nullptr) tma_store_2d(&p.tmD2, buf, n0, drow);
+        tma_store_2d(&p.tmD, buf + 2048, n0 >> 1, drow);
+      } else {
+        tma_store_2d(&p.tmD, buf, n0, drow);
+      }
+      tma_store_commit();
+      if (accum && c + 2 < chunk1) {
+        bulk_store_wait_read<0>();
+        fetch(c + 2);
+      }
+    }
+  }
+}
+
+// Epilogue of one warp for one output tile: the warp's 32 accumulator rows (TMEM lanes of its
+// quarter, BN fp32 columns starting at taddr0) go through bias / activation / residual / row map /
+// accumulate and are stored. `row_in_prob` is this thread's row within the problem; the warp
+// handles the 32-column chunks [chunk0, chunk1) (two warps share a lane quarter).
 template <int BN>
 __device__ __forceinline__ void epilogue_rows(const Problem& p, int M, int m0, int row_in_prob, int n_base,
-                                              uint32_t taddr0, int chunk0, int chunk1) {
+                                              uint32_t taddr0, int chunk0, int chunk1, uint8_t* stage, uint64_t* bar,
+                                              uint32_t& phase, volatile int* abort_flag) {
+  const int lane = threadIdx.x & 31;
+  const int row_first = warp_uniform(row_in_prob - lane);
+  if (p.tma_out && row_first + 32 <= M &&
+      WX_CHK(m0 >= 0 && m0 + row_first + 32 <= p.d_rows, 2009, m0 + row_first, p.d_rows)) {
+    epilogue_rows_tma<BN>(p, m0 + row_first, lane, n_base, taddr0, chunk0, chunk1, stage, bar, phase, abort_flag);
+    return;
+  }
   const bool row_ok = row_in_prob < M;
   long drow = static_cast<long>(m0) + row_in_prob;
   // Rows between M and the end of the 128-row tile are zero-filled on request, so that a
@@ -523,7 +727,9 @@ gemm_kernel(const __grid_constant__ GemmArgs args, int* __restrict__ status) {
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + C::STAGES * C::STAGE_BYTES);
+  uint8_t* epi_stage = smem + C::STAGES * C::STAGE_BYTES;
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(epi_stage + kEpiStage);
+  uint64_t* epi_bar = reinterpret_cast<uint64_t*>(epi_stage + kEpiStage + 256);
   uint64_t* empty_bar = full_bar + C::STAGES;
   uint64_t* tfull_bar = empty_bar + C::STAGES;
   uint64_t* tempty_bar = tfull_bar + 2;
@@ -547,6 +753,7 @@ gemm_kernel(const __grid_constant__ GemmArgs args, int* __restrict__ status) {
         mbar_init(&tfull_bar[a], 1);
         mbar_init(&tempty_bar[a], kEpiWarps);
       }
+      for (int w = 0; w < 2 * kEpiWarps; ++w) mbar_init(&epi_bar[w], 1);
     }
     *abort_flag = 0;
     fence_mbar_init();
@@ -682,6 +889,7 @@ gemm_kernel(const __grid_constant__ GemmArgs args, int* __restrict__ status) {
     constexpr int kChunks = BN / 32;
     const int chunk0 = (kChunks >= 2) ? half * (kChunks / 2) : 0;
     const int chunk1 = (kChunks >= 2) ? chunk0 + kChunks / 2 : (half == 0 ? 1 : 0);
+    uint32_t epi_phase = 0;
     int it = 0;
     for (int t = cta; t < total_tiles; t += ncta, ++it) {
       const TileInfo ti = decode_tile(d, t, gathered, rot0, rot1);
@@ -692,11 +900,13 @@ gemm_kernel(const __grid_constant__ GemmArgs args, int* __restrict__ status) {
       tc_fence_after();
 
       epilogue_rows<BN>(p, d.M[ti.prob], d.m0[ti.prob], ti.mt * BM + quarter * 32 + lane, ti.nt * BN,
-                        tmem_base + acc * BN + (static_cast<uint32_t>(quarter * 32) << 16), chunk0, chunk1);
+                        tmem_base + acc * BN + (static_cast<uint32_t>(quarter * 32) << 16), chunk0, chunk1,
+                        epi_stage + (warp - kEpiWarp0) * kEpiWarpStage, epi_bar + 2 * (warp - kEpiWarp0), epi_phase, abort_flag);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&tempty_bar[acc]);
     }
+    if (lane == 0) bulk_store_wait_all();
   }
 
   tc_fence_before();
@@ -740,7 +950,7 @@ void bind_context_once() {
 
 // 2-D bf16 tensor map with 128-byte swizzle; `inner` is the contiguous extent.
 bool make_tmap(CUtensorMap* out, const void* ptr, uint64_t inner, uint64_t outer, uint64_t pitch_elems,
-               uint32_t box_inner, uint32_t box_outer) {
+               uint32_t box_inner, uint32_t box_outer, CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_128B) {
   EncodeTiledFn fn = get_encode_fn();
   if (fn == nullptr) return false;
   bind_context_once();
@@ -749,7 +959,7 @@ bool make_tmap(CUtensorMap* out, const void* ptr, uint64_t inner, uint64_t outer
   cuuint32_t box[2] = {box_inner, box_outer};
   cuuint32_t estr[2] = {1, 1};
   CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, estr,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS;
 }
@@ -779,7 +989,7 @@ int launch_bn(const GemmArgs& args, bool a_mn, bool b_mn, int grid, cudaStream_t
   return launch_t<BN, true, true>(args, grid, stream, status);
 }
 
-int fill_args(GemmArgs& args, const GemmCall* calls, int ncalls, int bn, int a_rows = BM) {
+int fill_args(GemmArgs& args, const GemmCall* calls, int ncalls, int bn, int a_rows = BM, bool store_maps = true) {
   args.nprob = ncalls;
   {
     static const int env_group = [] {
@@ -822,6 +1032,24 @@ int fill_args(GemmArgs& args, const GemmCall* calls, int ncalls, int bn, int a_r
     p.m0 = c.m0;
     p.k0 = c.k0;
     p.flags = c.flags;
+    p.tma_out = 0;
+    const auto rows_ok = [](const void* q, long ld) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0 && (ld & 7) == 0; };
+    if (store_maps && !(c.flags & GEMM_OUT_FP32) && c.row_map == nullptr && c.d_rows >= 32 && rows_ok(c.D, c.ldd)) {
+      const bool swiglu = (c.flags & GEMM_ACT_SWIGLU) != 0, bwd = (c.flags & GEMM_SWIGLU_BWD) != 0;
+      bool maps;
+      if (bwd) {
+        maps = c.N % 32 == 0 && rows_ok(c.D2, c.ldd2) && c.bias == nullptr &&
+               make_tmap(&p.tmD, c.D, 2l * c.N, c.d_rows, c.ldd, 64, 32) && make_tmap(&p.tmD2, c.D2, 2l * c.N, c.d_rows, c.ldd2, 64, 32);
+      } else if (swiglu) {
+        maps = !(c.flags & GEMM_ACCUMULATE) && c.N % 32 == 0 &&
+               make_tmap(&p.tmD, c.D, c.N / 2, c.d_rows, c.ldd, 16, 32, CU_TENSOR_MAP_SWIZZLE_NONE);
+        if (maps && c.D2 != nullptr)
+          maps = rows_ok(c.D2, c.ldd2) && make_tmap(&p.tmD2, c.D2, c.N, c.d_rows, c.ldd2, 32, 32, CU_TENSOR_MAP_SWIZZLE_64B);
+      } else {
+        maps = make_tmap(&p.tmD, c.D, c.N, c.d_rows, c.ldd, 32, 32, CU_TENSOR_MAP_SWIZZLE_64B);
+      }
+      p.tma_out = maps ? 1 : 0;
+    }
   }
   return 0;
 }

@@ -26,7 +26,8 @@ constexpr int kPairStages = 6;
 constexpr int kPairABytes = BM * BK * 2;           // 128 rows of A, 64 k
 constexpr int kPairBBytes = 128 * BK * 2;          // this CTA's 128-row half of B
 constexpr int kPairStageBytes = kPairABytes + kPairBBytes;
-constexpr int kPairSmemBytes = kPairStages * kPairStageBytes + 1024 + 256;
+constexpr int kPairSmemBytes = kPairStages * kPairStageBytes + kEpiStage + 1024 + 256 + kEpiBarBytes;
+static_assert(kPairSmemBytes <= 227 * 1024, "stages and epilogue staging must fit");
 constexpr int kPairTileM = 2 * BM;
 constexpr int kPairTileN = 256;
 
@@ -46,7 +47,9 @@ gemm_pair_kernel(const __grid_constant__ GemmArgs args, int* __restrict__ status
   const int rot1 = (gathered && !B_MN) ? args.ag[1].rot : 0;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + kPairStages * kPairStageBytes);
+  uint8_t* epi_stage = smem + kPairStages * kPairStageBytes;
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(epi_stage + kEpiStage);
+  uint64_t* epi_bar = reinterpret_cast<uint64_t*>(epi_stage + kEpiStage + 256);
   uint64_t* empty_bar = full_bar + kPairStages;
   uint64_t* tfull_bar = empty_bar + kPairStages;
   uint64_t* tempty_bar = tfull_bar + 2;
@@ -70,6 +73,7 @@ gemm_pair_kernel(const __grid_constant__ GemmArgs args, int* __restrict__ status
         mbar_init(&tfull_bar[a], 1);   // one commit per tile, in each CTA
         mbar_init(&tempty_bar[a], 2 * kEpiWarps);  // used in the leader only: the epilogue warps of both CTAs
       }
+      for (int w = 0; w < 2 * kEpiWarps; ++w) mbar_init(&epi_bar[w], 1);
     }
     *abort_flag = 0;
     fence_mbar_init();
@@ -214,6 +218,7 @@ gemm_pair_kernel(const __grid_constant__ GemmArgs args, int* __restrict__ status
     const int quarter = warp & 3;
     const int half = (warp - kEpiWarp0) >> 2;  // two warps per lane quarter, half of the columns each
     const int chunk0 = half * (kPairTileN / 64), chunk1 = chunk0 + kPairTileN / 64;
+    uint32_t epi_phase = 0;
     int it = 0;
     for (int t = pair; t < total_tiles; t += npair, ++it) {
       const TileInfo ti = decode_tile(d, t, gathered, rot0, rot1);
@@ -225,7 +230,9 @@ gemm_pair_kernel(const __grid_constant__ GemmArgs args, int* __restrict__ status
       epilogue_rows<kPairTileN>(p, d.M[ti.prob], d.m0[ti.prob],
                                 ti.mt * kPairTileM + static_cast<int>(rank) * BM + quarter * 32 + lane,
                                 ti.nt * kPairTileN,
-                                tmem_base + acc * kPairTileN + (static_cast<uint32_t>(quarter * 32) << 16), chunk0, chunk1);
+                                tmem_base + acc * kPairTileN + (static_cast<uint32_t>(quarter * 32) << 16), chunk0, chunk1,
+                                epi_stage + (warp - kEpiWarp0) * kEpiWarpStage, epi_bar + 2 * (warp - kEpiWarp0), epi_phase,
+                                abort_flag);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) {
@@ -233,6 +240,7 @@ gemm_pair_kernel(const __grid_constant__ GemmArgs args, int* __restrict__ status
         else mbar_arrive_cluster(mapa_u32(smem_u32(&tempty_bar[acc]), 0));
       }
     }
+    if (lane == 0) bulk_store_wait_all();
   }
 
   tc_fence_before();

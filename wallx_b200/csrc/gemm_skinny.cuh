@@ -478,7 +478,7 @@ int launch_few(const GemmCall* calls, int ncalls, const FewShape& sh, cudaStream
   // the partial tile reuses the ring
   if (sh.stages < 2 || sh.nb * kFewBN * 4 > few_smem(sh) - kFewSmemExtra || few_smem(sh) > kFewSmemMax) return -12;
   GemmArgs args;
-  const int rc = fill_args(args, calls, ncalls, kFewBN, sh.nb);
+  const int rc = fill_args(args, calls, ncalls, kFewBN, sh.nb, false);
   if (rc != 0) return rc;
   QkvCache* qc = calls[0].qkv;
   if (qc != nullptr) {
